@@ -166,12 +166,15 @@ __device__ __forceinline__ void contract_quartet(const DevData& d, const double2
     }
 }
 
-// One quartet (bra pair P, ket pair Q): integrals, J/K digestion.
-// Lane-private updates go straight to A; the bra J block is returned in jab
-// (already weighted) for the warp reduction.
+// One quartet (bra pair P, ket pair Q): integrals, J/K digestion.  Every lane of the
+// warp calls; `in`: the lane has a quartet.  split = lb | len << 8: 2^lb neighbouring
+// lanes share the quartet; each contracts len of the bra's primitive pairs with all of
+// the ket's, they add their sums in a fixed tree and the first of them goes on.
+// Lane-private updates go straight to A; the bra J block is returned in jab (already
+// weighted) for the warp reduction.
 template <int La, int Lb, int Lc, int Ld, bool FP32>
-__device__ __forceinline__ void fock_quartet(const DevData& d, const double2* __restrict__ bt, int P, int Q,
-                                             double* jab_out, int* nq_done, int* np_done) {
+__device__ __forceinline__ void fock_quartet(const DevData& d, const double2* __restrict__ bt, int P, int Q, bool in,
+                                             int split, int lane, double* jab_out, int* nq_done, int* np_done) {
     using Cls = EriClass<La, Lb, Lc, Ld>;
     constexpr int NA = Cls::NA, NB = Cls::NB, NC = Cls::NC, ND = Cls::ND;
     constexpr int NE = Cls::NE, NF = Cls::NF, NAB = NA * NB;
@@ -185,8 +188,10 @@ __device__ __forceinline__ void fock_quartet(const DevData& d, const double2* __
     const double ct = d.pr_Y[P] * d.pr_Y[Q];
     // the CPU get2e's two tests (Y_P Y_Q > cut, then with DNmax): the work list may
     // have been built at a tighter cutoff than the one in force
-    if (!(ct > d.cut) || !(ct * dnmax > d.cut)) return;
-    ++*nq_done;
+    in = in && ct > d.cut && ct * dnmax > d.cut;
+    if (!in && (split & 0xff) == 0) return;
+    const int pps = d.pr_pps[P], b0 = (lane & ((1 << (split & 0xff)) - 1)) * (split >> 8);
+    const int bp0 = d.pr_pp0[P] + b0 * pps, bnp = in ? min(split >> 8, d.pr_npp[P] - b0) : 0;
 
     const double2 gp1 = d.pr_geo[3 * P + 1], gp2 = d.pr_geo[3 * P + 2];
     const double2 gq0 = d.pr_geo[3 * Q], gq1 = d.pr_geo[3 * Q + 1], gq2 = d.pr_geo[3 * Q + 2];
@@ -199,14 +204,23 @@ __device__ __forceinline__ void fock_quartet(const DevData& d, const double2* __
     if constexpr (FP32) {
         // mixed form: small-bound quartet, vertical recursion and contraction in FP32
         float accf[NE * NF];
-        contract_quartet<La, Lb, Lc, Ld, float>(d, bt, d.pr_pp0[P], d.pr_npp[P], d.pr_pps[P], d.pr_pp0[Q],
-                                                d.pr_npp[Q], d.pr_pps[Q], Cc, dnmax, true, mq, accf, np_done);
+        contract_quartet<La, Lb, Lc, Ld, float>(d, bt, bp0, bnp, pps, d.pr_pp0[Q], d.pr_npp[Q], d.pr_pps[Q], Cc,
+                                                dnmax, true, mq, accf, np_done);
 #pragma unroll
         for (int i = 0; i < NE * NF; ++i) acc[i] = (double)accf[i];
     } else {
-        contract_quartet<La, Lb, Lc, Ld>(d, bt, d.pr_pp0[P], d.pr_npp[P], d.pr_pps[P], d.pr_pp0[Q], d.pr_npp[Q],
-                                         d.pr_pps[Q], Cc, dnmax, true, mq, acc, np_done);
+        contract_quartet<La, Lb, Lc, Ld>(d, bt, bp0, bnp, pps, d.pr_pp0[Q], d.pr_npp[Q], d.pr_pps[Q], Cc, dnmax,
+                                         true, mq, acc, np_done);
     }
+    if (split & 0xff) {   // warp-uniform
+        __syncwarp();
+        const int lanes = 1 << (split & 0xff);
+        for (int o = 1; o < lanes; o <<= 1)
+#pragma unroll
+            for (int i = 0; i < NE * NF; ++i) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], o);
+        if (bnp <= 0 || (threadIdx.x & (lanes - 1))) return;   // the first lane of a quartet that passed
+    }
+    ++*nq_done;
 
     // bra HRR per ket column
     double t1[NF * NAB];
@@ -584,8 +598,8 @@ __device__ __forceinline__ const double2* class_boys_rows(const double2* __restr
 // 256-thread blocks can always launch).
 constexpr int kMaxLaneWarps = 8;
 
-// Work item: x = bra pair, y = first ket pair, z = number of kets (<= 32),
-// w = 1 for the mixed form's FP32 quartets.
+// Work item: x = bra pair, y = first ket pair, z = number of kets (<= 32 / the lanes
+// per quartet), w = how lanes share a quartet (fock_quartet's split).
 // FP32 = true: the mixed form's small-bound items (VRR and contraction in FP32),
 // compiled apart so that the FP64 items keep their register budget and vice versa.
 // One work item of a per-lane class (the warp's bra pair against up to 32 kets,
@@ -599,7 +613,8 @@ __device__ __forceinline__ void lane_item(const DevData& d, const double2* __res
 #pragma unroll
     for (int i = 0; i < NAB; ++i) jab[i] = 0.0;
     int nq = 0, np = 0;
-    if (lane < w.z) fock_quartet<La, Lb, Lc, Ld, FP32>(d, bt, w.x, w.y + lane, jab, &nq, &np);
+    const int k = lane >> (w.w & 0xff);   // the lane's ket
+    fock_quartet<La, Lb, Lc, Ld, FP32>(d, bt, w.x, w.y + min(k, w.z - 1), k < w.z, w.w, lane, jab, &nq, &np);
     if (d.stats) {
         const unsigned sq = __reduce_add_sync(0xffffffffu, (unsigned)nq);
         const unsigned sp = __reduce_add_sync(0xffffffffu, (unsigned)np);
@@ -722,7 +737,8 @@ fock_class_kernel_batch(const DevData* __restrict__ dl, const BatchSeg* __restri
 #pragma unroll
         for (int i = 0; i < NAB; ++i) jab[i] = 0.0;
         int nq = 0, np = 0;
-        if (lane < w.z) fock_quartet<La, Lb, Lc, Ld, FP32>(d, bt, w.x, w.y + lane, jab, &nq, &np);
+        const int k = lane >> (w.w & 0xff);   // the lane's ket
+    fock_quartet<La, Lb, Lc, Ld, FP32>(d, bt, w.x, w.y + min(k, w.z - 1), k < w.z, w.w, lane, jab, &nq, &np);
         if (d.exchange_only) continue;
         const int P = w.x;
         const int fa = d.q_f0[d.pr_qa[P]], fb = d.q_f0[d.pr_qb[P]];
@@ -1509,6 +1525,13 @@ static cudaError_t occupancy(int device, int ci, int part, int wpb, size_t smem,
         if (it != cache.end()) { *bps = it->second; return cudaSuccess; }
     }
     cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(bps, g_classes[ci].kernel(part == 1), 32 * wpb, smem);
+    // The per-lane kernels use no shared memory and live on L1 (psss is 17% slower at the
+    // largest shared carveout), but beside the cooperative classes an SM keeps their
+    // carveout unless a kernel asks for its own: 32 H2O / 6-31G* over four streams
+    // 12.71 ms without the request, 11.23 with it.
+    if (e == cudaSuccess && !g_classes[ci].coop)
+        e = cudaFuncSetAttribute(g_classes[ci].kernel(part == 1), cudaFuncAttributePreferredSharedMemoryCarveout,
+                                 cudaSharedmemCarveoutMaxL1);
     if (e == cudaSuccess) {
         std::lock_guard<std::mutex> g(mu);
         cache[key] = *bps;
@@ -1541,19 +1564,46 @@ static int class_launch_shape(qk_ctx* c, int ci) {
 
 static int finish_work(qk_ctx* c);
 
+// Lanes per quartet of a per-lane class of order M whose bra pairs have bnp primitive
+// pairs and whose kets have knp (fock_quartet's split).  A lane works through its
+// primitive quartets one after another (0.4 us each for ssss, 1.2 us for pppp): 1296 of
+// them for two pairs of 6-fold contracted s shells, 81 for any STO-3G quartet.  Where
+// the molecule does not give every lane of the GPU many quartets, that chain is the
+// class's time and lanes share it; the price is a digestion by one lane of each group.
+// The limit on the chain falls with the class's cost per primitive quartet and follows
+// the number of shells, not the screened lists: lists built at different cutoffs are
+// cut alike.  Whole builds (ms, * one after another) without a limit, with this rule and
+// with limits of 54, 27 and 9 for every class:
+//   H2O / STO-3G 0.158 0.069 0.106 0.080 0.063    4 H2O / STO-3G 0.136 0.064 0.097 0.081 0.075
+//   10 H2O / 6-31G* 1.19 0.95 0.93 0.99 1.06
+//   20 H2O / 6-31G*, density of a late cycle * 3.36 2.29 2.35 2.38 2.77
+//   32 H2O / 6-31G* * 11.7 11.7 12.0 12.5 14.9 (pppp alone 0.164 0.113 0.113 0.105 0.134)
+static int lane_split(int bnp, int knp, int M, int nq) {
+    const int chain = nq <= 10 ? 9 : nq <= 64 ? 40 : nq <= 256 ? 108 : 216;
+    const int limit = std::max(2 * chain / (2 + M), 1);
+    int lb = 0, len = bnp;
+    while (len > 1 && len * knp > limit && lb < 5) {
+        ++lb;
+        len = (bnp - 1) / (1 << lb) + 1;
+    }
+    return lb | len << 8;
+}
+static int split_kets(int split) { return 32 >> (split & 0xff); }
+
 // Work items of every class built on the host (the reference implementation of
 // the lists; the device builder, build_work_device, gives the same lists and is
 // the default except for sharded contexts).
 static int build_work(qk_ctx* c) {
     PairTable& T = c->pairs;
     const double cut = c->integralCutoff;
+    const int nq = (int)c->qsh.size();
     for (int ci = 0; ci < kNumClasses; ++ci) {
         const ClassEntry& ce = g_classes[ci];
         ClassWork& W = c->work[ci];
         W.items.clear();
         W.nquart = W.nprimq = W.nquart32 = 0;
         const bool same = (ce.La == ce.Lc && ce.Lb == ce.Ld);
-        struct Tmp { int4 it; long long cost; };
+        struct Tmp { int4 it; int fp32; long long cost; };
         std::vector<Tmp> tmp;
         for (int bb = 0; bb < (int)T.buckets.size(); ++bb) {
             const Bucket& B = T.buckets[bb];
@@ -1576,10 +1626,11 @@ static int build_work(qk_ctx* c) {
                     if (nk <= 0) continue;
                     W.nquart += nk;
                     W.nprimq += (long long)T.npp[P] * K.npa * K.npb * nk;
-                    // per-lane classes: up to 32 kets per warp item; cooperative classes
-                    // (one quartet per warp at a time): one ket per item, so that the
-                    // few, long quartets spread over many warps
-                    const int chunk = ce.coop ? 1 : 32;
+                    // per-lane classes: as many kets per warp item as it has lanes for;
+                    // cooperative classes (one quartet per warp at a time): one ket per
+                    // item, so that the few, long quartets spread over many warps
+                    const int split = ce.coop ? 0 : lane_split(B.npa * B.npb, K.npa * K.npb, ce.La + ce.Lb + ce.Lc + ce.Ld, nq);
+                    const int chunk = ce.coop ? 1 : split_kets(split);
                     // mixed form: kets with yp * yq below fp32_bound (a suffix, Y sorted
                     // descending) go to FP32 items; the cooperative classes stay FP64
                     int n64 = nk;
@@ -1592,16 +1643,15 @@ static int build_work(qk_ctx* c) {
                         n64 = a;
                     }
                     W.nquart32 += nk - n64;
-                    for (int s = 0; s < n64; s += chunk)
-                        tmp.push_back({make_int4(P, K.begin + s, std::min(chunk, n64 - s), 0), cost});
-                    for (int s = n64; s < nk; s += chunk)
-                        tmp.push_back({make_int4(P, K.begin + s, std::min(chunk, nk - s), 1), cost});
+                    for (int part = 0; part < 2; ++part)
+                        for (int s = part ? n64 : 0, e = part ? nk : n64; s < e; s += chunk)
+                            tmp.push_back({make_int4(P, K.begin + s, std::min(chunk, e - s), split), part, cost});
                 }
             }
         }
         // FP64 items first, then the FP32 ones (two launches); each part by cost
         std::stable_sort(tmp.begin(), tmp.end(), [](const Tmp& x, const Tmp& y) {
-            if (x.it.w != y.it.w) return x.it.w < y.it.w;
+            if (x.fp32 != y.fp32) return x.fp32 < y.fp32;
             return x.cost > y.cost;
         });
         // a shard keeps every shard_count-th item of the cost-ordered list (each
@@ -1615,11 +1665,11 @@ static int build_work(qk_ctx* c) {
             for (const Tmp& t : tmp) {
                 W.nquart += t.it.z;
                 W.nprimq += t.cost * t.it.z;
-                if (t.it.w == 1) W.nquart32 += t.it.z;
+                if (t.fp32) W.nquart32 += t.it.z;
             }
         }
         W.n64 = 0;
-        for (const Tmp& t : tmp) W.n64 += t.it.w == 0;
+        for (const Tmp& t : tmp) W.n64 += t.fp32 == 0;
         W.items.resize(tmp.size());
         for (size_t i = 0; i < tmp.size(); ++i) W.items[i] = tmp[i].it;
         W.n_items = (int)W.items.size();
@@ -1678,12 +1728,12 @@ struct WlSeg {
     int bra0, bra1;        // bra pairs [bra0, bra1)
     int ket0, ket1;        // ket bucket [ket0, ket1), Y descending
     int ci;                // class
-    int chunk;             // kets per item: 32 (per-lane classes) or 1 (cooperative)
+    int chunk;             // kets per item: as many as split leaves lanes for (per-lane classes) or 1
     int tri;               // bra and ket bucket are the same: kets Q <= P only
     int fp32_ok;           // the mixed form may put this segment's small-bound kets in FP32 items
     long long ket_npp;     // primitive pairs of one ket pair
     int t0;                // first thread of the segment
-    int pad;
+    int split;             // lanes per quartet of the segment's items (fock_quartet)
 };
 
 __device__ __forceinline__ int wl_find_seg(const WlSeg* __restrict__ segs, int nseg, int t) {
@@ -1756,9 +1806,9 @@ __global__ void wl_emit_kernel(const WlSeg* __restrict__ segs, int nseg, int nth
     const int n64 = n64_in[t];
     const int first = cls[3 * sg.ci], base = cls[3 * sg.ci + 1], n64c = cls[3 * sg.ci + 2];
     int4* o = items + base + (off64[t] - off64[first]);
-    for (int k = 0; k < n64; k += sg.chunk) *o++ = make_int4(P, sg.ket0 + k, min(sg.chunk, n64 - k), 0);
+    for (int k = 0; k < n64; k += sg.chunk) *o++ = make_int4(P, sg.ket0 + k, min(sg.chunk, n64 - k), sg.split);
     o = items + base + n64c + (off32[t] - off32[first]);
-    for (int k = n64; k < nk; k += sg.chunk) *o++ = make_int4(P, sg.ket0 + k, min(sg.chunk, nk - k), 1);
+    for (int k = n64; k < nk; k += sg.chunk) *o++ = make_int4(P, sg.ket0 + k, min(sg.chunk, nk - k), sg.split);
 }
 
 static size_t wl_align(size_t x) { return (x + 255) & ~(size_t)255; }
@@ -1768,6 +1818,7 @@ static size_t wl_align(size_t x) { return (x + 255) & ~(size_t)255; }
 static int build_work_device(qk_ctx* c) {
     PairTable& T = c->pairs;
     cudaStream_t s = c->stream;
+    const int nq = (int)c->qsh.size();
     // segments, class by class, each class's in build_work's item order
     std::vector<WlSeg> segs;
     std::vector<int> ct0(kNumClasses), ct1(kNumClasses);
@@ -1789,6 +1840,8 @@ static int build_work_device(qk_ctx* c) {
                 sg.ci = ci; sg.chunk = ce.coop ? 1 : 32; sg.tri = (same && kb == bb) ? 1 : 0;
                 sg.fp32_ok = ce.coop ? 0 : 1;
                 sg.ket_npp = (long long)K.npa * K.npb;
+                sg.split = ce.coop ? 0 : lane_split(B.npa * B.npb, K.npa * K.npb, ce.La + ce.Lb + ce.Lc + ce.Ld, nq);
+                if (!ce.coop) sg.chunk = split_kets(sg.split);
                 cand.push_back({sg, (long long)B.npa * B.npb * K.npa * K.npb});
             }
         }
