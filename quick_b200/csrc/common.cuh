@@ -80,30 +80,57 @@ __device__ __forceinline__ void boys_scaled(double T, double scale, const double
     }
 }
 
-// Boys table F_m(k * dT), m < kBoysNM, from the convergent series
-// F_m(T) = exp(-T) sum_k (2T)^k / ((2m+1)(2m+3)...(2m+2k+1)) in long double.
-// F_0..F_M at T from a per-M row table (kBoysNT rows of 8 doubles: F_M..F_{M+6}
-// at T_k, then exp(-T_k)): the same arithmetic as boys_scaled, with four 16-byte
-// loads of one 64-byte row per evaluation instead of eight 8-byte ones.
-constexpr int kBoysRow = 8;
+// F_0..F_M at T from the class's row table, one row per grid point, read with 16-byte
+// loads, up to boys_tmax(M); above it exp(-T) changes no F_m, m <= M, by 2^-54 of its
+// value and the asymptotic form F_m = (2m-1)!!/(2T)^m sqrt(pi/T)/2 is exact to rounding.
+// Nearly every warp has lanes on both sides of the line, so both branches are paid for:
+// with the line at 36 for every M the second one needed an exponential and a division
+// and the evaluation was 47% of psss's instructions and 52% of its FP64 ones.
+//   M = 0: 48-byte rows, the six coefficients of F_0's Chebyshev interpolation on
+//          intervals of 1/32 (truncation 1.7e-16 relative); no exponential is needed.
+//   M > 0: 80-byte rows, F_{M+j}(T_k)/j! for j = 0..6 (Taylor, spacing 0.05) and
+//          exp(-T_k) for the downward recursion; the last two words are padding.
+// Both strides are odd multiples of 16 bytes: 32 lanes on random rows then spread over
+// all eight 16-byte bank groups of L1 (41 SM cycles a warp for four loads against 82
+// with 64-byte rows, which start in two of the groups).
+constexpr int kBoysRow0 = 6, kBoysRow = 10;      // doubles per row, M = 0 and M > 0
+__host__ __device__ constexpr int boys_tmax(int M) {
+    constexpr int t[13] = {36, 40, 44, 47, 50, 53, 56, 59, 61, 64, 66, 69, 71};
+    return M < 13 ? t[M] : 71 + 3 * (M - 12);
+}
+__host__ __device__ constexpr int boys_nrow(int M) { return boys_tmax(M) * (M == 0 ? 32 : 20) + 1; }
+__host__ __device__ constexpr size_t boys_rows_at(int M) {   // first double of M's rows
+    size_t at = 0;
+    for (int m = 0; m < M; ++m) at += ((size_t)boys_nrow(m) * (m == 0 ? kBoysRow0 : kBoysRow) + 1) / 2 * 2;
+    return at;
+}
 template <int M>
 __device__ __forceinline__ void boys_scaled_rows(double T, double scale, const double2* __restrict__ rows,
                                                  double* F) {
-    if (T < kBoysTmax) {
-        const int k = __double2int_rn(T * kBoysInvDT);
-        const double u = k * kBoysDT - T;
-        const double2* r = rows + k * (kBoysRow / 2);
-        const double2 c01 = __ldg(r), c23 = __ldg(r + 1), c45 = __ldg(r + 2), c6e = __ldg(r + 3);
-        double f = c6e.x * (1.0 / 720.0);
-        f = fma(f, u, c45.y * (1.0 / 120.0));
-        f = fma(f, u, c45.x * (1.0 / 24.0));
-        f = fma(f, u, c23.y * (1.0 / 6.0));
-        f = fma(f, u, c23.x * 0.5);
-        f = fma(f, u, c01.y);
-        f = fma(f, u, c01.x);
-        if (M == 0) {
+    if (T < (double)boys_tmax(M)) {
+        if constexpr (M == 0) {
+            const int k = __double2int_rn(T * 32.0);
+            const double u = fma((double)k, -0.03125, T);
+            const double2* r = rows + k * (kBoysRow0 / 2);
+            const double2 c01 = __ldg(r), c23 = __ldg(r + 1), c45 = __ldg(r + 2);
+            double f = fma(c45.y, u, c45.x);
+            f = fma(f, u, c23.y);
+            f = fma(f, u, c23.x);
+            f = fma(f, u, c01.y);
+            f = fma(f, u, c01.x);
             F[0] = f * scale;
         } else {
+            const int k = __double2int_rn(T * kBoysInvDT);
+            const double u = k * kBoysDT - T;
+            const double2* r = rows + k * (kBoysRow / 2);
+            const double2 c01 = __ldg(r), c23 = __ldg(r + 1), c45 = __ldg(r + 2), c6e = __ldg(r + 3);
+            double f = fma(c6e.x, u, c45.y);
+            f = fma(f, u, c45.x);
+            f = fma(f, u, c23.y);
+            f = fma(f, u, c23.x);
+            f = fma(f, u, c01.y);
+            f = fma(f, u, c01.x);
+            // exp(-T) = exp(-T_k) exp(u)
             double eu = fma(u, 1.0 / 720.0, 1.0 / 120.0);
             eu = fma(eu, u, 1.0 / 24.0);
             eu = fma(eu, u, 1.0 / 6.0);
@@ -121,16 +148,16 @@ __device__ __forceinline__ void boys_scaled_rows(double T, double scale, const d
             }
         }
     } else {
-        double f0 = kHalfSqrtPi * rsqrt(T);
-        F[0] = f0 * scale;
-        if (M > 0) {
-            const double e = exp(-T);
-            const double h = 0.5 / T;
-            double fm = f0;
+        const double r = rsqrt(T);
+        double fm = kHalfSqrtPi * r * scale;
+        F[0] = fm;
+        if constexpr (M > 0) {
+            double h = 0.5 * r * r;             // 1/(2T), one Newton step to full precision
+            h = fma(h, fma(-2.0 * T, h, 1.0), h);
 #pragma unroll
             for (int m = 0; m < M; ++m) {
-                fm = fma((double)(2 * m + 1), fm, -e) * h;
-                F[m + 1] = fm * scale;
+                fm *= (double)(2 * m + 1) * h;
+                F[m + 1] = fm;
             }
         }
     }
@@ -245,37 +272,85 @@ __device__ __forceinline__ double boys_quick_one(int m, int M, double X) {
     return f;
 }
 
-// Row tables for M = 0 .. 4 kMaxL from boys_table(): block M holds kBoysNT rows
-// of kBoysRow doubles (F_M..F_{M+6}, exp(-T_k)).
+// F_m(T) from the convergent series
+// F_m(T) = exp(-T) sum_k (2T)^k / ((2m+1)(2m+3)...(2m+2k+1)) in long double.
+inline long double boys_series(int m, long double T) {
+    long double term = 1.0L / (2 * m + 1), sum = term;
+    for (int j = 1; j < 4000; ++j) {
+        term *= 2.0L * T / (2 * m + 2 * j + 1);
+        sum += term;
+        if (fabsl(term) < sum * 1e-22L) break;
+    }
+    return expl(-T) * sum;
+}
+
+// Row tables of boys_scaled_rows: M = 0, then M = 1 .. 4 kMaxL from boys_table().
 inline std::vector<double> boys_row_tables(const std::vector<double>& tab) {
     const int nM = 4 * kMaxL + 1;
-    std::vector<double> r((size_t)nM * kBoysNT * kBoysRow);
-    for (int M = 0; M < nM; ++M)
-        for (int k = 0; k < kBoysNT; ++k) {
-            double* row = &r[((size_t)M * kBoysNT + k) * kBoysRow];
-            for (int j = 0; j < 7; ++j) row[j] = tab[(size_t)k * kBoysNM + M + j];
-            row[7] = tab[(size_t)kBoysNT * kBoysNM + k];
+    std::vector<double> r(boys_rows_at(nM), 0.0);
+    // M = 0: interpolation of F_0 at the six Chebyshev nodes of each interval, as a
+    // Chebyshev sum and then in powers of u
+    const int n = kBoysRow0;
+    const long double half = 1.0L / 64.0L, pi = 3.141592653589793238462643383279502884L;
+    for (int k = 0; k < boys_nrow(0); ++k) {
+        long double f[n], c[n], a[n] = {};
+        for (int i = 0; i < n; ++i) {
+            long double T = k / 32.0L + half * cosl(pi * (i + 0.5L) / n);
+            // left of zero the series alternates but converges as fast (|T| <= 1/64)
+            f[i] = boys_series(0, T);
+        }
+        for (int j = 0; j < n; ++j) {
+            c[j] = 0.0L;
+            for (int i = 0; i < n; ++i) c[j] += f[i] * cosl(pi * j * (i + 0.5L) / n);
+            c[j] *= (j ? 2.0L : 1.0L) / n;
+        }
+        long double t0[n] = {1.0L}, t1[n] = {0.0L, 1.0L};   // T_{j-1}, T_j in powers of x
+        for (int i = 0; i < n; ++i) a[i] = c[0] * t0[i] + c[1] * t1[i];
+        for (int j = 2; j < n; ++j) {
+            long double t2[n] = {};
+            for (int i = 0; i < n; ++i) t2[i] = (i ? 2.0L * t1[i - 1] : 0.0L) - t0[i];
+            for (int i = 0; i < n; ++i) {
+                a[i] += c[j] * t2[i];
+                t0[i] = t1[i];
+                t1[i] = t2[i];
+            }
+        }
+        long double s = 1.0L;   // x = u / half
+        for (int i = 0; i < n; ++i) {
+            r[(size_t)k * n + i] = (double)(a[i] * s);
+            s /= half;
+        }
+    }
+    for (int M = 1; M < nM; ++M)
+        for (int k = 0; k < boys_nrow(M); ++k) {
+            double* row = &r[boys_rows_at(M) + (size_t)k * kBoysRow];
+            double fact = 1.0;
+            for (int j = 0; j < 7; ++j) {
+                fact *= j > 1 ? j : 1;
+                // the plain table ends at kBoysTmax
+                row[j] = (k < kBoysNT ? tab[(size_t)k * kBoysNM + M + j]
+                                      : (double)boys_series(M + j, k * (long double)kBoysDT)) / fact;
+            }
+            row[7] = (double)expl(-k * (long double)kBoysDT);
         }
     return r;
 }
 
+// Boys table F_m(k * dT), m < kBoysNM, then exp(-k * dT).
 inline std::vector<double> boys_table() {
     std::vector<double> t((size_t)kBoysNT * kBoysNM);
     for (int k = 0; k < kBoysNT; ++k) {
         long double T = (long double)k * kBoysDT;
         for (int m = 0; m < kBoysNM; ++m) {
-            long double term = 1.0L / (2 * m + 1), sum = term;
-            for (int j = 1; j < 4000; ++j) {
-                term *= 2.0L * T / (2 * m + 2 * j + 1);
-                sum += term;
-                if (term < sum * 1e-22L) break;
-            }
-            t[(size_t)k * kBoysNM + m] = (double)(expl(-T) * sum);
+            t[(size_t)k * kBoysNM + m] = (double)boys_series(m, T);
         }
     }
     // exp(-T_k) after the table (used for the downward recursion)
     for (int k = 0; k < kBoysNT; ++k) t.push_back((double)expl(-(long double)k * kBoysDT));
     return t;
 }
+
+// The tables above in a device's memory (get2e.cu).
+cudaError_t device_boys_tables(int device, cudaStream_t s, const double** tab, const double** rows);
 
 }  // namespace qk

@@ -583,13 +583,10 @@ fock_coop_kernel(DevData d, const int4* __restrict__ items, int n_items, int* __
     }
 }
 
-// The class's Boys row table (kBoysNT rows of 64 bytes): an evaluation reads one
-// row with four 16-byte loads, served from L1 for the hot part of the T range.
-// (Staging the 46 KB table in shared memory costs more in occupancy than it
-// saves in load latency: measured 1.8x slower on the ssss class.)
+// The class's Boys row table (boys_scaled_rows).
 template <int M>
 __device__ __forceinline__ const double2* class_boys_rows(const double2* __restrict__ src) {
-    return src + (size_t)M * kBoysNT * (kBoysRow / 2);
+    return src + boys_rows_at(M) / 2;
 }
 
 // Per-lane class kernels launch with 1..kMaxLaneWarps warps per block (default
@@ -860,7 +857,7 @@ schwarz_kernel(DevData d, const int2* __restrict__ work, int n_work, const int* 
     if (mode >= 0) { p0 += mode * ps; np = 1; }
     double acc[NE * NF];
     int ndone = 0;
-    contract_quartet<La, Lb, La, Lb>(d, d.boys8 + (size_t)Cls::M * kBoysNT * (kBoysRow / 2), p0, np, ps, p0, np, ps,
+    contract_quartet<La, Lb, La, Lb>(d, class_boys_rows<Cls::M>(d.boys8), p0, np, ps, p0, np, ps,
                                      Cc, 0.0, false, 2 * (d.q_ltop[qa] + d.q_ltop[qb]), acc, &ndone);
     double t1[NF * NAB];
 #pragma unroll
@@ -1017,7 +1014,7 @@ __global__ void boys_probe_kernel(const double* __restrict__ T, int n, const dou
     if (mode)
         boys_quick_scaled<M>(T[i], 1.0, F, M);
     else
-        boys_scaled_rows<M>(T[i], 1.0, rows8 + (size_t)M * kBoysNT * (kBoysRow / 2), F);
+        boys_scaled_rows<M>(T[i], 1.0, class_boys_rows<M>(rows8), F);
 #pragma unroll
     for (int m = 0; m <= M; ++m) {
         f_rows[(size_t)i * (M + 1) + m] = F[m];
@@ -1269,7 +1266,8 @@ struct qk_ctx {
     int last_launches = 0;             // kernel launches of the last build
     int num_sms = 148;
     // device buffers
-    qk::DevBuf<double> d_xyz, d_boys, d_boys8, d_D, d_cutmat, d_o;
+    qk::DevBuf<double> d_xyz, d_D, d_cutmat, d_o;
+    const double *boys = nullptr, *boys_rows = nullptr;   // the device's tables (device_boys_tables)
     qk::DevBuf<int> d_q_atom, d_q_f0, d_q_parent, d_q_ltop, d_q_prim0, d_q_nprim, d_shell_f0, d_shell_f1;
     qk::DevBuf<unsigned long long> d_A, d_A2;   // d_A2: the exchange-only half of a UHF build
     qk::DevBuf<double> d_uhf;                     // UHF: Dt and Ds (2 nbasis^2), then Db and ob for host calls
@@ -1366,8 +1364,8 @@ static DevData make_devdata(qk_ctx* c) {
     d.pp_pxy = c->pairs.d_pxy.p;
     d.pp_pzax = c->pairs.d_pzax.p;
     d.pp_payz = c->pairs.d_payz.p;
-    d.boys = c->d_boys.p;
-    d.boys8 = (const double2*)c->d_boys8.p;
+    d.boys = c->boys;
+    d.boys8 = (const double2*)c->boys_rows;
     d.cut = c->integralCutoff;
     d.primLimit = c->primLimit;
     d.boys_mode = c->boys_mode;
@@ -2352,6 +2350,44 @@ int qk_set_maxprim(int maxprim) {
 
 int qk_max_l(void) { return kMaxL; }
 
+}  // extern "C"
+
+namespace qk {
+// The Boys tables (boys_table, boys_row_tables) in the device's memory: the same for
+// every context, so made once per device at its first context and kept.
+cudaError_t device_boys_tables(int device, cudaStream_t s, const double** tab, const double** rows) {
+    static std::mutex mu;
+    static double* tables[64] = {};
+    static std::vector<double> host;
+    static size_t rows_at = 0;
+    if (device < 0 || device >= 64) return cudaErrorInvalidDevice;
+    std::lock_guard<std::mutex> g(mu);
+    if (host.empty()) {
+        host = boys_table();
+        const std::vector<double> r = boys_row_tables(host);
+        if (host.size() % 2) host.push_back(0.0);   // rows are read 16 bytes at a time
+        rows_at = host.size();
+        host.insert(host.end(), r.begin(), r.end());
+    }
+    if (!tables[device]) {
+        double* p = nullptr;
+        cudaError_t e = cudaMalloc((void**)&p, host.size() * sizeof(double));
+        if (e == cudaSuccess) e = cudaMemcpyAsync(p, host.data(), host.size() * sizeof(double), cudaMemcpyHostToDevice, s);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+        if (e != cudaSuccess) {
+            if (p) cudaFree(p);
+            return e;
+        }
+        tables[device] = p;
+    }
+    *tab = tables[device];
+    *rows = tables[device] + rows_at;
+    return cudaSuccess;
+}
+}  // namespace qk
+
+extern "C" {
+
 qk_ctx* qk_create(int device, int* status) {
     int ndev = 0;
     if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) {
@@ -2380,15 +2416,7 @@ qk_ctx* qk_create(int device, int* status) {
         if (status) *status = fail(QK_ERR_CUDA, "stream creation failed");
         return nullptr;
     }
-    // the tables are the same for every context: computed once per process
-    static std::once_flag once;
-    static std::vector<double> tab, rows;
-    std::call_once(once, [] {
-        tab = boys_table();
-        rows = boys_row_tables(tab);
-    });
-    if (c->d_boys.upload(tab, c->stream) != cudaSuccess || c->d_boys8.upload(rows, c->stream) != cudaSuccess ||
-        cudaStreamSynchronize(c->stream) != cudaSuccess) {
+    if (device_boys_tables(device, c->stream, &c->boys, &c->boys_rows) != cudaSuccess) {
         cudaStreamDestroy(c->stream);
         delete c;
         if (status) *status = fail(QK_ERR_CUDA, "Boys table upload failed");
@@ -2944,7 +2972,7 @@ int qk_device_bytes(qk_ctx* c, unsigned long long* total, unsigned long long* it
     unsigned long long t = it;
     for (size_t b : {T.d_qa.bytes(), T.d_qb.bytes(), T.d_pp0.bytes(), T.d_npp.bytes(), T.d_pps.bytes(),
                      T.d_Y.bytes(), T.d_zo.bytes(), T.d_kc.bytes(), T.d_pxy.bytes(), T.d_pzax.bytes(),
-                     T.d_payz.bytes(), T.d_sh.bytes(), T.d_lt.bytes(), T.d_geo.bytes(), c->d_xyz.bytes(), c->d_boys.bytes(), c->d_boys8.bytes(), c->d_schwarz_Y.bytes(), c->d_schwarz_cp.bytes(), c->d_D.bytes(), c->d_cutmat.bytes(),
+                     T.d_payz.bytes(), T.d_sh.bytes(), T.d_lt.bytes(), T.d_geo.bytes(), c->d_xyz.bytes(), c->d_schwarz_Y.bytes(), c->d_schwarz_cp.bytes(), c->d_D.bytes(), c->d_cutmat.bytes(),
                      c->d_o.bytes(), c->d_q_atom.bytes(), c->d_q_f0.bytes(), c->d_q_parent.bytes(), c->d_q_ltop.bytes(),
                      c->d_q_prim0.bytes(), c->d_q_nprim.bytes(), c->d_shell_f0.bytes(), c->d_shell_f1.bytes(),
                      c->d_A.bytes(), c->d_A2.bytes(), c->d_uhf.bytes(), c->d_counters.bytes(), c->d_stats.bytes()})
@@ -3136,8 +3164,8 @@ int qk_boys(qk_ctx* c, int M, const double* T, int n, double* F_rows, double* F_
     QK_CUDA_TRY(dr.reserve(nout));
     QK_CUDA_TRY(d1.reserve(nout));
     QK_CUDA_TRY(cudaMemcpyAsync(dT.p, T, sizeof(double) * n, cudaMemcpyHostToDevice, s));
-    const double2* rows8 = (const double2*)c->d_boys8.p;
-    const double* tab = c->d_boys.p;
+    const double2* rows8 = (const double2*)c->boys_rows;
+    const double* tab = c->boys;
     cudaError_t e = cudaErrorInvalidValue;
     switch (M) {
 #define QK_BOYS_CASE(m) case m: e = launch_boys_probe<m>(dT.p, n, rows8, tab, c->boys_mode, dr.p, d1.p, s); break;

@@ -322,7 +322,7 @@ oei_shell_kernel(OeiArgs a, const int4* __restrict__ pairs, int chunk, const dou
     const double* B = a.xyz + 3 * (a.ncenter[fb0] - 1);
     const double AB[3] = {A[0] - B[0], A[1] - B[1], A[2] - B[2]};
     const double r2 = AB[0] * AB[0] + AB[1] * AB[1] + AB[2] * AB[2];
-    const double2* bt = rows + (size_t)L * kBoysNT * (kBoysRow / 2);
+    const double2* bt = rows + boys_rows_at(L) / 2;
     double acc[NOUT];
 #pragma unroll
     for (int k = 0; k < NOUT; ++k) acc[k] = 0.0;
@@ -450,52 +450,29 @@ static cudaStream_t oei_stream(int device) {
     return streams[device];
 }
 
-// Per device, made at the first call and kept: the Boys tables in device memory (the
-// plain table, then the row tables), and a memory pool of its own for the calls' work
-// buffers, which keeps up to 256 MB between calls instead of giving the pages back to
-// the driver at every synchronisation.
-struct OeiDevice {
-    double* boys = nullptr;
-    size_t rows_at = 0;        // doubles
-    cudaMemPool_t pool = nullptr;
-    bool ready = false;
-};
-static int oei_device(int device, cudaStream_t s, OeiDevice* out) {
+// Per device, made at the first call and kept: a memory pool of its own for the calls'
+// work buffers, which keeps up to 256 MB between calls instead of giving the pages back
+// to the driver at every synchronisation.
+static cudaMemPool_t oei_pool(int device) {
     static std::mutex mu;
-    static OeiDevice dev[64];
-    if (device < 0 || device >= 64) return QK_ERR_INVALID_ARG;
+    static cudaMemPool_t pools[64] = {};
+    if (device < 0 || device >= 64) return nullptr;
     std::lock_guard<std::mutex> g(mu);
-    OeiDevice& d = dev[device];
-    if (!d.ready) {
-        std::vector<double> tab = boys_table();
-        const std::vector<double> rows = boys_row_tables(tab);
-        if (tab.size() % 2) tab.push_back(0.0);   // the rows start on a 16-byte boundary
-        d.rows_at = tab.size();
-        tab.insert(tab.end(), rows.begin(), rows.end());
-        if (!d.boys && cudaMalloc((void**)&d.boys, tab.size() * 8) != cudaSuccess) {
-            d.boys = nullptr;
-            return QK_ERR_OUT_OF_MEMORY;
+    if (!pools[device]) {
+        cudaMemPoolProps props{};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = device;
+        unsigned long long keep = 256ull << 20;
+        cudaMemPool_t p = nullptr;
+        if (cudaMemPoolCreate(&p, &props) != cudaSuccess) return nullptr;
+        if (cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+            cudaMemPoolDestroy(p);
+            return nullptr;
         }
-        if (cudaMemcpyAsync(d.boys, tab.data(), tab.size() * 8, cudaMemcpyHostToDevice, s) != cudaSuccess ||
-            cudaStreamSynchronize(s) != cudaSuccess)
-            return QK_ERR_CUDA;
-        if (!d.pool) {
-            cudaMemPoolProps props{};
-            props.allocType = cudaMemAllocationTypePinned;
-            props.location.type = cudaMemLocationTypeDevice;
-            props.location.id = device;
-            unsigned long long keep = 256ull << 20;
-            if (cudaMemPoolCreate(&d.pool, &props) != cudaSuccess) {
-                d.pool = nullptr;
-                return QK_ERR_CUDA;
-            }
-            if (cudaMemPoolSetAttribute(d.pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess)
-                return QK_ERR_CUDA;
-        }
-        d.ready = true;
+        pools[device] = p;
     }
-    *out = d;
-    return QK_OK;
+    return pools[device];
 }
 
 }  // namespace qk
@@ -576,9 +553,11 @@ extern "C" int qk_oei_host(int device, int natom, const double* xyz, const doubl
     chunk = (nq + nchunk - 1) / nchunk;
     cudaStream_t s = oei_stream(device);
     if (!s) return QK_ERR_CUDA;
-    OeiDevice dev;
-    int st = oei_device(device, s, &dev);
-    if (st != QK_OK) return st;
+    const double *boys = nullptr, *rows = nullptr;
+    if (device_boys_tables(device, s, &boys, &rows) != cudaSuccess) return QK_ERR_CUDA;
+    cudaMemPool_t pool = oei_pool(device);
+    if (!pool) return QK_ERR_CUDA;
+    int st = QK_OK;
     // one device block: inputs (packed on the host, one copy), then S T V, then the
     // partial sums
     std::vector<int4> sp_all;
@@ -600,7 +579,7 @@ extern "C" int qk_oei_host(int device, int natom, const double* xyz, const doubl
     for (int i = 0; i < 9; ++i)
         if (sizes[i] > 0) std::memcpy(packed.data() + off[i], src[i], sizes[i]);
     char* base = nullptr;
-    if (cudaMallocFromPoolAsync((void**)&base, total, dev.pool, s) != cudaSuccess) return QK_ERR_OUT_OF_MEMORY;
+    if (cudaMallocFromPoolAsync((void**)&base, total, pool, s) != cudaSuccess) return QK_ERR_OUT_OF_MEMORY;
     if (cudaMemcpyAsync(base, packed.data(), packed.size(), cudaMemcpyHostToDevice, s) != cudaSuccess) st = QK_ERR_CUDA;
     if (st == QK_OK) {
         OeiArgs a;
@@ -609,18 +588,17 @@ extern "C" int qk_oei_host(int device, int natom, const double* xyz, const doubl
         a.aexp = (const double*)(base + off[2]); a.dcoeff = (const double*)(base + off[3]);
         a.ncenter = (const int*)(base + off[4]); a.xyz = (const double*)(base + off[5]);
         a.cxyz = (const double*)(base + off[6]); a.cq = (const double*)(base + off[7]);
-        a.boys = dev.boys;
+        a.boys = boys;
         a.S = (double*)(base + off[9]); a.T = a.S + nn; a.V = a.T + nn;
         double* Vpart = (double*)(base + off[10]);
         const int gx = (int)((npair + 127) / 128);
         oei_st_kernel<<<gx, 128, 0, s>>>(a);
         if (shells) {
             const int4* dsp = (const int4*)(base + off[8]);
-            const double2* rows = (const double2*)(dev.boys + dev.rows_at);
 #define QK_OEI_SP(LA, LB)                                                                              \
             if (!sp_list[LA][LB].empty())                                                              \
                 oei_shell_kernel<LA, LB><<<dim3((unsigned)sp_list[LA][LB].size(), nchunk), threads, 0, s>>>( \
-                    a, dsp + sp_off[LA][LB], chunk, rows, Vpart);
+                    a, dsp + sp_off[LA][LB], chunk, (const double2*)rows, Vpart);
             // the longest blocks first
             QK_OEI_SP(3, 3) QK_OEI_SP(3, 2) QK_OEI_SP(3, 1) QK_OEI_SP(2, 2) QK_OEI_SP(3, 0) QK_OEI_SP(2, 1)
             QK_OEI_SP(2, 0) QK_OEI_SP(1, 1) QK_OEI_SP(1, 0) QK_OEI_SP(0, 0)

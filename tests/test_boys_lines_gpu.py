@@ -1,0 +1,41 @@
+"""GPU test of the Boys row tables at the places where a class's evaluation changes: the
+line between table and asymptote (36 for M = 0, up to 71 for M = 12), the last rows
+below it and the rows past the plain table's end at 36, against mpmath."""
+import ctypes
+
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+from test_boys_gpu import _boys_mp  # noqa: E402
+
+LINES = [36, 40, 44, 47, 50, 53, 56, 59, 61, 64, 66, 69, 71]
+
+
+@pytest.mark.parametrize("M", range(13))
+def test_boys_rows_at_the_lines(M):
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from quick_b200._native import check, lib
+    from quick_b200.basis import build_basis
+    from quick_b200.get2e import Get2e
+    from quick_b200.molecules import water_cluster
+    L = lib()
+    if M > 4 * L.qk_max_l():
+        pytest.skip("M above the compiled maximum")
+    t = float(LINES[M])
+    T = np.concatenate([[0.0, 1.0 / 64, np.nextafter(1.0 / 64, 1), 0.024999, 0.025001, np.nextafter(t, 0), t, t + 1e-9,
+                         t - 0.0249, t - 0.0251, t - 1.0 / 64, 35.99, 36.01], np.linspace(30.0, 80.0, 41)])
+    eng = Get2e(build_basis(water_cluster(1, 3.0), "STO-3G"))
+    n = len(T)
+    Fr, F1 = np.zeros((n, M + 1)), np.zeros((n, M + 1))
+    P = lambda a: ctypes.c_void_p(a.ctypes.data)  # noqa: E731
+    check(L.qk_boys(ctypes.c_void_p(eng.h), M, P(T), n, P(Fr), P(F1)), "qk_boys")
+    eng.close()
+    for i, x in enumerate(T):
+        for m in range(M + 1):
+            ref = float(_boys_mp(m, float(x)))
+            # a table value at 1.5e-15 (M = 12) and at most 2M + 2 roundings of a recursion
+            assert abs(Fr[i, m] - ref) <= (1.5e-15 + (2 * M + 2) * 1.2e-16) * ref, (M, m, x)
