@@ -98,6 +98,15 @@ __device__ __forceinline__ double warp_sum(double v) {
     return v;
 }
 
+// The class kernels of a build do not depend on one another (their sums meet in integer
+// atomics), but they follow one another in a stream, and each one's last blocks leave
+// most of the GPU idle: 21 kernels for s, p and d shells, 55 with f.  They are therefore
+// launched as programmatic dependents (launch_kernel): each lets the next one's blocks
+// in as its own leave, and ends only after the kernel before it has, so that whatever
+// follows the last one in the stream follows them all.
+__device__ __forceinline__ void class_kernel_begin() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void class_kernel_end() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // Contracted [e0|f0] over the primitive pairs of a bra and a ket pair.
 // acc[f*NE + e]; prim_screen applies QUICK's primitive cutoff.  R is the type of
 // the vertical recursion and of acc: double for the plain path, float for the
@@ -568,6 +577,7 @@ fock_coop_kernel(DevData d, const int4* __restrict__ items, int n_items, int* __
     double* acc = smem + (size_t)warp * Lay::PER_WARP;
     double* V = acc + Lay::ACC;
     double* Db = V + Lay::WORK;
+    class_kernel_begin();
     for (;;) {
         int it = 0;
         if (lane == 0) it = atomicAdd(counter, 1);
@@ -581,6 +591,7 @@ fock_coop_kernel(DevData d, const int4* __restrict__ items, int n_items, int* __
             atomicAdd(d.stats + 1, (unsigned long long)np);
         }
     }
+    class_kernel_end();
 }
 
 // The class's Boys row table (boys_scaled_rows).
@@ -638,6 +649,7 @@ fock_class_kernel(DevData d, const int4* __restrict__ items, int n_items, int* _
     using Cls = EriClass<La, Lb, Lc, Ld>;
     const int lane = threadIdx.x & 31;
     const double2* bt = class_boys_rows<Cls::M>(d.boys8);
+    class_kernel_begin();
     for (;;) {
         int it = 0;
         if (lane == 0) it = atomicAdd(counter, 1);
@@ -645,6 +657,7 @@ fock_class_kernel(DevData d, const int4* __restrict__ items, int n_items, int* _
         if (it >= n_items) break;
         lane_item<La, Lb, Lc, Ld, FP32>(d, bt, items[it], lane);
     }
+    class_kernel_end();
 }
 
 // The s/p classes in one persistent kernel (qk_set_merge_sp): the six per-lane s/p
@@ -667,6 +680,7 @@ __global__ void __launch_bounds__(32 * kMaxLaneWarps)
 fock_merged_sp_kernel(DevData d, const MergedSeg* __restrict__ segs, int nseg, int n_items,
                       int* __restrict__ counter) {
     const int lane = threadIdx.x & 31;
+    class_kernel_begin();
     for (;;) {
         int it = 0;
         if (lane == 0) it = atomicAdd(counter, 1);
@@ -688,6 +702,7 @@ fock_merged_sp_kernel(DevData d, const MergedSeg* __restrict__ segs, int nseg, i
             default: lane_item<0, 0, 0, 0, FP32>(d, class_boys_rows<EriClass<0, 0, 0, 0>::M>(d.boys8), w, lane); break;
         }
     }
+    class_kernel_end();
 }
 #endif
 
@@ -722,6 +737,7 @@ fock_class_kernel_batch(const DevData* __restrict__ dl, const BatchSeg* __restri
     constexpr int NAB = Cls::NA * Cls::NB;
     const int lane = threadIdx.x & 31;
     const double2* bt = class_boys_rows<Cls::M>(dl[0].boys8);
+    class_kernel_begin();
     for (;;) {
         int it = 0;
         if (lane == 0) it = atomicAdd(counter, 1);
@@ -746,6 +762,7 @@ fock_class_kernel_batch(const DevData* __restrict__ dl, const BatchSeg* __restri
                 atomic_fixed(d.A + (size_t)(fa + i / Cls::NB) * d.nbasis + fb + i % Cls::NB, s);
         }
     }
+    class_kernel_end();
 }
 
 template <int La, int Lb, int Lc, int Ld>
@@ -758,6 +775,7 @@ fock_coop_kernel_batch(const DevData* __restrict__ dl, const BatchSeg* __restric
     double* acc = smem + (size_t)warp * Lay::PER_WARP;
     double* V = acc + Lay::ACC;
     double* Db = V + Lay::WORK;
+    class_kernel_begin();
     for (;;) {
         int it = 0;
         if (lane == 0) it = atomicAdd(counter, 1);
@@ -769,6 +787,7 @@ fock_coop_kernel_batch(const DevData* __restrict__ dl, const BatchSeg* __restric
         int nq = 0, np = 0;
         for (int k = 0; k < w.z; ++k) coop_quartet<La, Lb, Lc, Ld>(d, w.x, w.y + k, acc, V, Db, lane, &nq, &np);
     }
+    class_kernel_end();
 }
 
 // The per-lane kernels of the s/p classes, single-molecule and batched, FP64 and FP32.
@@ -1140,16 +1159,33 @@ struct PairTable {
     }
 };
 
-using FockFn = void (*)(bool, dim3, dim3, size_t, cudaStream_t, const DevData&, const int4*, int, int*);
+// Launches a class kernel; `after`: as a programmatic dependent of the class kernel before
+// it in the stream (class_kernel_begin).
+template <typename... P, typename... A>
+static void launch_kernel(void (*k)(P...), bool after, dim3 g, dim3 bl, size_t smem, cudaStream_t s, A... a) {
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = g;
+    cfg.blockDim = bl;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = &at;
+    cfg.numAttrs = after ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, k, static_cast<P>(a)...);   // an error stays for cudaGetLastError
+}
+
+using FockFn = void (*)(bool, bool, dim3, dim3, size_t, cudaStream_t, const DevData&, const int4*, int, int*);
 template <int a, int b, int c, int e>
-void launch_fock(bool fp32, dim3 g, dim3 bl, size_t smem, cudaStream_t s, const DevData& dd, const int4* it, int n,
+void launch_fock(bool fp32, bool after, dim3 g, dim3 bl, size_t smem, cudaStream_t s, const DevData& dd, const int4* it, int n,
                  int* cnt) {
     if constexpr (EriClass<a, b, c, e>::COOP)
-        fock_coop_kernel<a, b, c, e><<<g, bl, smem, s>>>(dd, it, n, cnt);
+        launch_kernel(&fock_coop_kernel<a, b, c, e>, after, g, bl, smem, s, dd, it, n, cnt);
     else if (fp32)
-        fock_class_kernel<a, b, c, e, true><<<g, bl, smem, s>>>(dd, it, n, cnt);
+        launch_kernel(&fock_class_kernel<a, b, c, e, true>, after, g, bl, smem, s, dd, it, n, cnt);
     else
-        fock_class_kernel<a, b, c, e, false><<<g, bl, smem, s>>>(dd, it, n, cnt);
+        launch_kernel(&fock_class_kernel<a, b, c, e, false>, after, g, bl, smem, s, dd, it, n, cnt);
 }
 template <int a, int b, int c, int e>
 const void* fock_fn_ptr(bool fp32) {
@@ -1160,16 +1196,16 @@ const void* fock_fn_ptr(bool fp32) {
     else
         return (const void*)&fock_class_kernel<a, b, c, e, false>;
 }
-using FockBatchFn = void (*)(bool, dim3, dim3, size_t, cudaStream_t, const DevData*, const BatchSeg*, int, int, int*);
+using FockBatchFn = void (*)(bool, bool, dim3, dim3, size_t, cudaStream_t, const DevData*, const BatchSeg*, int, int, int*);
 template <int a, int b, int c, int e>
-void launch_fock_batch(bool fp32, dim3 g, dim3 bl, size_t smem, cudaStream_t s, const DevData* dl,
+void launch_fock_batch(bool fp32, bool after, dim3 g, dim3 bl, size_t smem, cudaStream_t s, const DevData* dl,
                        const BatchSeg* segs, int nseg, int n, int* cnt) {
     if constexpr (EriClass<a, b, c, e>::COOP)
-        fock_coop_kernel_batch<a, b, c, e><<<g, bl, smem, s>>>(dl, segs, nseg, n, cnt);
+        launch_kernel(&fock_coop_kernel_batch<a, b, c, e>, after, g, bl, smem, s, dl, segs, nseg, n, cnt);
     else if (fp32)
-        fock_class_kernel_batch<a, b, c, e, true><<<g, bl, smem, s>>>(dl, segs, nseg, n, cnt);
+        launch_kernel(&fock_class_kernel_batch<a, b, c, e, true>, after, g, bl, smem, s, dl, segs, nseg, n, cnt);
     else
-        fock_class_kernel_batch<a, b, c, e, false><<<g, bl, smem, s>>>(dl, segs, nseg, n, cnt);
+        launch_kernel(&fock_class_kernel_batch<a, b, c, e, false>, after, g, bl, smem, s, dl, segs, nseg, n, cnt);
 }
 template <int a, int b, int c, int e>
 const void* fock_batch_fn_ptr(bool fp32) {
@@ -1562,8 +1598,8 @@ static int class_launch_shape(qk_ctx* c, int ci) {
 
 static int finish_work(qk_ctx* c);
 
-// Lanes per quartet of a per-lane class of order M whose bra pairs have bnp primitive
-// pairs and whose kets have knp (fock_quartet's split).  A lane works through its
+// Lanes per quartet of a per-lane class whose bra pairs have bnp primitive pairs and
+// whose kets have knp (fock_quartet's split).  A lane works through its
 // primitive quartets one after another (0.4 us each for ssss, 1.2 us for pppp): 1296 of
 // them for two pairs of 6-fold contracted s shells, 81 for any STO-3G quartet.  Where
 // the molecule does not give every lane of the GPU many quartets, that chain is the
@@ -1576,9 +1612,10 @@ static int finish_work(qk_ctx* c);
 //   10 H2O / 6-31G* 1.19 0.95 0.93 0.99 1.06
 //   20 H2O / 6-31G*, density of a late cycle * 3.36 2.29 2.35 2.38 2.77
 //   32 H2O / 6-31G* * 11.7 11.7 12.0 12.5 14.9 (pppp alone 0.164 0.113 0.113 0.105 0.134)
-static int lane_split(int bnp, int knp, int M, int nq) {
+static int lane_split(int bnp, int knp, double prim_flops, int nq) {
     const int chain = nq <= 10 ? 9 : nq <= 64 ? 40 : nq <= 256 ? 108 : 216;
-    const int limit = std::max(2 * chain / (2 + M), 1);
+    // a primitive quartet takes a lane about 0.35 us + 1.1 ns per operation
+    const int limit = std::max((int)(chain * 0.41 / (0.35 + 1.1e-3 * prim_flops)), 1);
     int lb = 0, len = bnp;
     while (len > 1 && len * knp > limit && lb < 5) {
         ++lb;
@@ -1627,7 +1664,7 @@ static int build_work(qk_ctx* c) {
                     // per-lane classes: as many kets per warp item as it has lanes for;
                     // cooperative classes (one quartet per warp at a time): one ket per
                     // item, so that the few, long quartets spread over many warps
-                    const int split = ce.coop ? 0 : lane_split(B.npa * B.npb, K.npa * K.npb, ce.La + ce.Lb + ce.Lc + ce.Ld, nq);
+                    const int split = ce.coop ? 0 : lane_split(B.npa * B.npb, K.npa * K.npb, ce.prim_flops, nq);
                     const int chunk = ce.coop ? 1 : split_kets(split);
                     // mixed form: kets with yp * yq below fp32_bound (a suffix, Y sorted
                     // descending) go to FP32 items; the cooperative classes stay FP64
@@ -1838,7 +1875,7 @@ static int build_work_device(qk_ctx* c) {
                 sg.ci = ci; sg.chunk = ce.coop ? 1 : 32; sg.tri = (same && kb == bb) ? 1 : 0;
                 sg.fp32_ok = ce.coop ? 0 : 1;
                 sg.ket_npp = (long long)K.npa * K.npb;
-                sg.split = ce.coop ? 0 : lane_split(B.npa * B.npb, K.npa * K.npb, ce.La + ce.Lb + ce.Lc + ce.Ld, nq);
+                sg.split = ce.coop ? 0 : lane_split(B.npa * B.npb, K.npa * K.npb, ce.prim_flops, nq);
                 if (!ce.coop) sg.chunk = split_kets(sg.split);
                 cand.push_back({sg, (long long)B.npa * B.npb * K.npa * K.npb});
             }
@@ -2011,13 +2048,14 @@ static int prepare_merged(qk_ctx* c) {
 
 // One class's launches: its FP64 items, then (mixed form) its FP32 items, each
 // part with its own counter (counters[ci] and counters[kNumClasses + ci]).
+// after: a class kernel of this build is the last thing in the stream (launch_kernel).
 static void launch_class(const ClassEntry& ce, const ClassWork& W, cudaStream_t s, const DevData& d, int* counters,
-                         int ci) {
+                         int ci, bool after) {
     const int n = W.n_items;
     if (W.n64 > 0)
-        ce.fn(false, dim3(W.grid), dim3(W.block), W.smem, s, d, W.d_items, W.n64, counters + ci);
+        ce.fn(false, after, dim3(W.grid), dim3(W.block), W.smem, s, d, W.d_items, W.n64, counters + ci);
     if (n > W.n64)
-        ce.fn(true, dim3(W.grid32), dim3(W.block), W.smem, s, d, W.d_items + W.n64, n - W.n64,
+        ce.fn(true, after || W.n64 > 0, dim3(W.grid32), dim3(W.block), W.smem, s, d, W.d_items + W.n64, n - W.n64,
               counters + kNumClasses + ci);
 }
 
@@ -2069,6 +2107,7 @@ static int fock2e_device(qk_ctx* c, const double* D, const double* cutmat, doubl
     // remaining SMs).  With per-class event timing on they run one after another
     // on `s`, so that every class kernel is timed alone.
     const bool concurrent = !c->profile_events && c->nstreams > 0;
+    bool on_s = false;   // a class kernel is the last thing in `s`
 #if QK_MAX_L >= 1
     if (merged) {
         // the joined s/p lists first, on the caller's stream
@@ -2076,13 +2115,11 @@ static int fock2e_device(qk_ctx* c, const double* D, const double* cutmat, doubl
             if (c->m_items[part] > 0) {
                 const MergedSeg* sg = c->d_mseg.p + (part ? c->m_nseg[0] : 0);
                 int* ctr = c->d_counters.p + 2 * kNumClasses + part;
-                if (part)
-                    fock_merged_sp_kernel<true><<<c->m_grid[1], c->m_block, 0, s>>>(d, sg, c->m_nseg[1],
-                                                                                  c->m_items[1], ctr);
-                else
-                    fock_merged_sp_kernel<false><<<c->m_grid[0], c->m_block, 0, s>>>(d, sg, c->m_nseg[0],
-                                                                                   c->m_items[0], ctr);
+                launch_kernel(part ? &fock_merged_sp_kernel<true> : &fock_merged_sp_kernel<false>, on_s,
+                              dim3(c->m_grid[part]), dim3(c->m_block), 0, s, d, sg, c->m_nseg[part], c->m_items[part],
+                              ctr);
                 QK_CUDA_TRY(cudaGetLastError());
+                on_s = !c->profile_events;
             }
     }
 #endif
@@ -2097,9 +2134,11 @@ static int fock2e_device(qk_ctx* c, const double* D, const double* cutmat, doubl
             continue;
         }
         cudaStream_t ls = s;
+        bool after = on_s;
         if (concurrent) {
             const int k = slot++ % c->nstreams;
             ls = c->aux[k];
+            after = used[k];
             if (!used[k]) {
                 QK_CUDA_TRY(cudaStreamWaitEvent(ls, c->fork_ev, 0));
                 used[k] = true;
@@ -2108,8 +2147,9 @@ static int fock2e_device(qk_ctx* c, const double* D, const double* cutmat, doubl
         if (c->profile_stats) d.stats = c->d_stats.p + 2 * ci;
         if (c->profile_events) QK_CUDA_TRY(cudaEventRecord(c->ev[2 * ci], ls));
         const ClassEntry& ce = g_classes[ci];
-        launch_class(ce, W, ls, d, c->d_counters.p, ci);
+        launch_class(ce, W, ls, d, c->d_counters.p, ci, after);
         QK_CUDA_TRY(cudaGetLastError());
+        if (!concurrent) on_s = !c->profile_events;   // timed classes run alone
         if (c->profile_events) {
             QK_CUDA_TRY(cudaEventRecord(c->ev[2 * ci + 1], ls));
             c->ev_recorded[ci] = true;
@@ -2258,6 +2298,7 @@ static int fock2e_device_noalloc(qk_ctx* c, const double* D, const double* cutma
     // the launch shape of fock2e_device: concurrent over the context's nstreams
     // auxiliary streams, or one class after another on `s` (nstreams 0)
     const bool concurrent = c->nstreams > 0;
+    bool on_s = false;   // a class kernel is the last thing in `s`
     if (concurrent) QK_CUDA_TRY(cudaEventRecord(c->fork_ev, s));
     bool used[qk_ctx::kAux] = {};
     int slot = 0;
@@ -2265,17 +2306,20 @@ static int fock2e_device_noalloc(qk_ctx* c, const double* D, const double* cutma
     for (int ci : c->launch_order) {
         const ClassWork& W = c->work[ci];
         cudaStream_t ls = s;
+        bool after = on_s;
         if (concurrent) {
             const int k = slot++ % c->nstreams;
             ls = c->aux[k];
+            after = used[k];
             if (!used[k]) {
                 QK_CUDA_TRY(cudaStreamWaitEvent(ls, c->fork_ev, 0));
                 used[k] = true;
             }
         }
         const ClassEntry& ce = g_classes[ci];
-        launch_class(ce, W, ls, d, counters, ci);
+        launch_class(ce, W, ls, d, counters, ci, after);
         QK_CUDA_TRY(cudaGetLastError());
+        if (!concurrent) on_s = true;
         nq += W.nquart;
         npq += W.nprimq;
     }
@@ -2945,7 +2989,7 @@ int qk_batch_fock2e(qk_batch* b, int n, qk_ctx* const* ctxs, const double* const
         const long long need = ((long long)total_items[slot] + wpb - 1) / wpb;
         const int sms = std::max(1, b->num_sms - b->reserve_sms);
         const int grid = (int)std::min<long long>((long long)b->bps[slot] * sms, need);
-        ce.fn_batch(slot >= kNumClasses, dim3(grid), dim3(32 * wpb), ce.smem, s, dd, dg + seg_off[slot],
+        ce.fn_batch(slot >= kNumClasses, i > 0, dim3(grid), dim3(32 * wpb), ce.smem, s, dd, dg + seg_off[slot],
                     seg_count[slot], total_items[slot], b->d_counters.p + slot);
         QK_CUDA_TRY(cudaGetLastError());
     }

@@ -32,9 +32,10 @@ def test_shared_quartets_match_oracle(bas, nw, bound):
     eng.set_precision(bound)
     got = eng.fock2e(torch.tensor(D, device="cuda")).cpu().numpy()
     eng.close()
-    # FP64: the accumulator's 2^-45 a term over at most 2 n^2 terms, and FP64 sums of
-    # |G| ~ 100 (1e-13 relative); mixed: quartets below the bound at FP32's 6e-8
-    tol = 2 * b.nbasis * 2.0 ** -45 + 1e-13 * np.abs(want).max()
+    # FP64: an element sums at most n^2 Coulomb and n^2 exchange terms, twice (A + A^T),
+    # each rounded to 2^-45, and FP64 sums of |G| (1e-13 relative); mixed: quartets below
+    # the bound at FP32's 6e-8
+    tol = 4 * b.nbasis ** 2 * 2.0 ** -45 + 1e-13 * np.abs(want).max()
     if bound:
         tol += bound * 6e-8 * b.nbasis
     assert np.abs(got - want).max() <= tol
