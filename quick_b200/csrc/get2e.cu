@@ -1606,12 +1606,14 @@ static int finish_work(qk_ctx* c);
 // class's time and lanes share it; the price is a digestion by one lane of each group.
 // The limit on the chain falls with the class's cost per primitive quartet and follows
 // the number of shells, not the screened lists: lists built at different cutoffs are
-// cut alike.  Whole builds (ms, * one after another) without a limit, with this rule and
-// with limits of 54, 27 and 9 for every class:
+// cut alike.  Whole builds (ms, * one after another) without a limit, with this rule by
+// the class's order, and with limits of 54, 27 and 9 for every class:
 //   H2O / STO-3G 0.158 0.069 0.106 0.080 0.063    4 H2O / STO-3G 0.136 0.064 0.097 0.081 0.075
 //   10 H2O / 6-31G* 1.19 0.95 0.93 0.99 1.06
 //   20 H2O / 6-31G*, density of a late cycle * 3.36 2.29 2.35 2.38 2.77
 //   32 H2O / 6-31G* * 11.7 11.7 12.0 12.5 14.9 (pppp alone 0.164 0.113 0.113 0.105 0.134)
+// By the operations instead of the order, the long d classes alone are cut finer: dppp of
+// 10 H2O 0.105 -> 0.087, of the late cycle 0.201 -> 0.177.
 static int lane_split(int bnp, int knp, double prim_flops, int nq) {
     const int chain = nq <= 10 ? 9 : nq <= 64 ? 40 : nq <= 256 ? 108 : 216;
     // a primitive quartet takes a lane about 0.35 us + 1.1 ns per operation
