@@ -101,9 +101,11 @@ __device__ __forceinline__ double warp_sum(double v) {
 // The class kernels of a build do not depend on one another (their sums meet in integer
 // atomics), but they follow one another in a stream, and each one's last blocks leave
 // most of the GPU idle: 21 kernels for s, p and d shells, 55 with f.  They are therefore
-// launched as programmatic dependents (launch_kernel): each lets the next one's blocks
-// in as its own leave, and ends only after the kernel before it has, so that whatever
-// follows the last one in the stream follows them all.
+// launched as programmatic dependents (launch_kernel): once all of a kernel's blocks have
+// started, the next one's take whatever room there is beside them and the room that they
+// leave, and a kernel ends only after the one before it has, so that whatever follows the
+// last one in the stream follows them all.  A grid that is kept small to leave SMs to other
+// work (qk_batch_reserve_sms) is launched plainly: the next kernel would fill those SMs.
 __device__ __forceinline__ void class_kernel_begin() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void class_kernel_end() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
@@ -2991,8 +2993,9 @@ int qk_batch_fock2e(qk_batch* b, int n, qk_ctx* const* ctxs, const double* const
         const long long need = ((long long)total_items[slot] + wpb - 1) / wpb;
         const int sms = std::max(1, b->num_sms - b->reserve_sms);
         const int grid = (int)std::min<long long>((long long)b->bps[slot] * sms, need);
-        ce.fn_batch(slot >= kNumClasses, i > 0, dim3(grid), dim3(32 * wpb), ce.smem, s, dd, dg + seg_off[slot],
-                    seg_count[slot], total_items[slot], b->d_counters.p + slot);
+        // with SMs reserved one class kernel at a time (class_kernel_begin)
+        ce.fn_batch(slot >= kNumClasses, i > 0 && b->reserve_sms == 0, dim3(grid), dim3(32 * wpb), ce.smem, s, dd,
+                    dg + seg_off[slot], seg_count[slot], total_items[slot], b->d_counters.p + slot);
         QK_CUDA_TRY(cudaGetLastError());
     }
     batch_finalize_kernel<<<dim3(chunks, n), 256, 0, s>>>(dm);

@@ -5,6 +5,8 @@ launch per class, so every molecule sees exactly the quartets (and the int64
 accumulation order does not matter) of its own one-molecule build: the results
 must equal ``qk_fock2e_device`` bit for bit, and those are checked against the
 oracle in the one-molecule tests."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -131,3 +133,40 @@ def test_batch_many_small_molecules():
     bt.close()
     for e in engs:
         e.close()
+
+
+class _Edge(ctypes.Structure):   # CUgraphEdgeData
+    _fields_ = [("from_port", ctypes.c_ubyte), ("to_port", ctypes.c_ubyte), ("type", ctypes.c_ubyte),
+                ("reserved", ctypes.c_ubyte * 5)]
+
+
+def _programmatic_edges(graph):
+    """How many edges of a captured graph let a kernel start before the one it follows has ended."""
+    get = ctypes.CDLL("libcuda.so.1").cuGraphGetEdges_v2
+    h, n = ctypes.c_void_p(graph.raw_cuda_graph()), ctypes.c_size_t(0)
+    assert get(h, None, None, None, ctypes.byref(n)) == 0
+    a, b, e = (ctypes.c_void_p * n.value)(), (ctypes.c_void_p * n.value)(), (_Edge * n.value)()
+    assert get(h, a, b, e, ctypes.byref(n)) == 0
+    return sum(x.type == 1 for x in e)   # CU_GRAPH_DEPENDENCY_TYPE_PROGRAMMATIC
+
+
+@pytest.mark.parametrize("reserve", [0, 8])
+def test_reserved_sms_stay_free(engines, reserve):
+    """A reserved batch's grids leave SMs free only while one class kernel runs at a time: none of them may be let in
+    beside the one before it.  The launches are looked at in a captured graph (which is not replayed)."""
+    from quick_b200.get2e import Get2eBatch
+    singles = [e.fock2e(D).cpu().numpy() for _, e, D in engines]
+    bt = Get2eBatch()
+    bt.reserve_sms(reserve)
+    got = bt.fock2e([e for _, e, _ in engines], [D for _, _, D in engines])
+    for (name, _, _), s, g in zip(engines, singles, got):
+        assert g.cpu().numpy().tobytes() == s.tobytes(), name
+    bt.close()
+    bt = Get2eBatch()   # a batch that has recorded no event outside the capture
+    bt.reserve_sms(reserve)
+    g = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(g, capture_error_mode="relaxed"):
+        bt.fock2e([e for _, e, _ in engines], [D for _, _, D in engines], os=got)
+    assert (_programmatic_edges(g) > 0) == (reserve == 0)
+    del g
+    bt.close()
