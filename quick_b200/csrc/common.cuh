@@ -152,8 +152,11 @@ __device__ __forceinline__ void boys_scaled_rows(double T, double scale, const d
         double fm = kHalfSqrtPi * r * scale;
         F[0] = fm;
         if constexpr (M > 0) {
-            double h = 0.5 * r * r;             // 1/(2T), one Newton step to full precision
-            h = fma(h, fma(-2.0 * T, h, 1.0), h);
+            // 1/(2T), one Newton step to full precision; T = infinity (a distance whose square
+            // overflows) counts as the largest number in it, so that h stays 0 and not inf * 0
+            const double rr = r * r, tf = __hiloint2double(min(__double2hiint(T), 0x7fefffff), __double2loint(T));
+            double h = 0.5 * rr;
+            h = fma(h, fma(-tf, rr, 1.0), h);
 #pragma unroll
             for (int m = 0; m < M; ++m) {
                 fm *= (double)(2 * m + 1) * h;

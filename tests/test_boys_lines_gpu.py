@@ -39,3 +39,39 @@ def test_boys_rows_at_the_lines(M):
             ref = float(_boys_mp(m, float(x)))
             # a table value at 1.5e-15 (M = 12) and at most 2M + 2 roundings of a recursion
             assert abs(Fr[i, m] - ref) <= (1.5e-15 + (2 * M + 2) * 1.2e-16) * ref, (M, m, x)
+
+
+def _boys_rows(M, T):
+    """F_0..F_M at every T by the per-lane kernels' evaluation, one row per T."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from quick_b200._native import check, lib
+    from quick_b200.basis import build_basis
+    from quick_b200.get2e import Get2e
+    from quick_b200.molecules import water_cluster
+    L = lib()
+    if M > 4 * L.qk_max_l():
+        pytest.skip("M above the compiled maximum")
+    eng = Get2e(build_basis(water_cluster(1, 3.0), "STO-3G"))
+    n = len(T)
+    Fr, F1 = np.zeros((n, M + 1)), np.zeros((n, M + 1))
+    P = lambda a: ctypes.c_void_p(a.ctypes.data)  # noqa: E731
+    check(L.qk_boys(ctypes.c_void_p(eng.h), M, P(T), n, P(Fr), P(F1)), "qk_boys")
+    eng.close()
+    return Fr
+
+
+@pytest.mark.parametrize("M", range(13))
+def test_boys_rows_at_the_end_of_the_range(M):
+    """F_m = (2m-1)!!/(2T)^m sqrt(pi/T)/2 to where T overflows; at infinity every F_m is 0, as its limit is."""
+    T = np.array([1e10, 1e100, 1e200, 1e300, 8.9e307, 9.1e307, 1.7e308, np.inf])
+    Fr = _boys_rows(M, T)
+    assert np.all(Fr[-1] == 0.0)
+    assert np.all(np.isfinite(Fr))
+    with np.errstate(under="ignore", over="ignore"):
+        want = np.sqrt(np.pi / T) / 2
+        for m in range(M + 1):
+            # rsqrt is good to 2^-52, its factor and product add two roundings; a step has two and 1/(2T) to
+            # two; products under 2^-1022 lose digits
+            assert np.all(np.abs(Fr[:, m] - want) <= (4 + 4 * m) * 2.0 ** -53 * want + m * 2.0 ** -1022), m
+            want = want * ((2 * m + 1) / (2 * T))

@@ -47,3 +47,14 @@ def test_oei_takes_components_in_any_order(bas):
         setattr(q, f, np.asfortranarray(getattr(b, f)[:, p]))
     for got, want in zip(oei(q, ext), oei(b, ext)):
         assert np.abs(got - want[np.ix_(p, p)]).max() <= 1e-12 * max(1.0, np.abs(want).max())
+
+
+def test_oei_charge_beyond_the_range_adds_nothing():
+    """A charge so far away that its squared distance overflows."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from quick_b200.scf import oei
+    b = build_basis(water_cluster(2, 6.0, seed=2), "6-31G*")
+    far = (np.array([[1e155, 0.0, 0.0], [0.0, -3e160, 1e158]]), np.array([1.0, -2.0]))
+    for got, want in zip(oei(b, far), oei(b, None)):
+        assert np.array_equal(got, want)
