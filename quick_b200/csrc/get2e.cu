@@ -2411,8 +2411,9 @@ cudaError_t device_boys_tables(int device, cudaStream_t s, const double** tab, c
     if (device < 0 || device >= 64) return cudaErrorInvalidDevice;
     std::lock_guard<std::mutex> g(mu);
     if (host.empty()) {
-        host = boys_table();
-        const std::vector<double> r = boys_row_tables(host);
+        const std::vector<long double> grid = boys_grid();
+        host = boys_table(grid);
+        const std::vector<double> r = boys_row_tables(grid);
         if (host.size() % 2) host.push_back(0.0);   // rows are read 16 bytes at a time
         rows_at = host.size();
         host.insert(host.end(), r.begin(), r.end());

@@ -75,3 +75,20 @@ def test_boys_rows_at_the_end_of_the_range(M):
             # two; products under 2^-1022 lose digits
             assert np.all(np.abs(Fr[:, m] - want) <= (4 + 4 * m) * 2.0 ** -53 * want + m * 2.0 ** -1022), m
             want = want * ((2 * m + 1) / (2 * T))
+
+
+@pytest.mark.parametrize("M", [6, 8, 10, 12])
+def test_boys_rows_low_orders_keep_their_precision(M):
+    """The downward recursion may add one rounding a step to F_0, no more."""
+    T = np.random.default_rng(M).uniform(0.0, 90.0, 8000)
+    t, ref = T.astype(np.longdouble), np.zeros(len(T), dtype=np.longdouble)
+    term = np.ones(len(T), dtype=np.longdouble)
+    for j in range(1, 500):   # exp(T) F_0 = sum (2T)^j / (2j+1)!!
+        ref += term
+        term = term * (2 * t / (2 * j + 1))
+    ref *= np.exp(-t)
+    rms = float(np.sqrt(np.mean(((_boys_rows(M, T)[:, 0] - ref) / ref).astype(float) ** 2)))
+    # a rounding's relative error is 4.71e-17 rms (uniform in the last place, significands
+    # spread over their logarithm); the M steps and at most seven others: the table, the
+    # interpolation's last steps, the scale
+    assert rms <= 4.71e-17 * (M + 7) ** 0.5, rms
