@@ -58,3 +58,49 @@ def test_lane_split_does_not_depend_on_the_cutoff():
     assert torch.equal(eng.fock2e(D), want)
     fresh.close()
     eng.close()
+
+
+def _rounded_elements(b):
+    """How many rounded terms each element of the accumulator collects, every shell quartet of the basis taken: the
+    two Coulomb blocks and each element of the exchange blocks once."""
+    shells = []
+    for s in range(b.nshell):
+        for L in range(int(b.qstart[s]), int(b.qfinal[s]) + 1):
+            f0 = int(b.ksumtype[s]) - 1 + int(b.qsbasis[s, L])
+            shells.append(slice(f0, f0 + (L + 1) * (L + 2) // 2))
+    N = np.zeros((b.nbasis, b.nbasis))
+    pairs = [(x, y) for i, x in enumerate(shells) for y in shells[:i + 1]]
+    for i, (x, y) in enumerate(pairs):
+        for z, w in pairs[:i + 1]:
+            N[x, y] += 1
+            N[z, w] += 1
+            for u, v in {(x.start, z.start): (x, z), (y.start, z.start): (y, z), (x.start, w.start): (x, w),
+                         (y.start, w.start): (y, w)}.values():
+                N[u, v] += 1
+    return N
+
+
+@pytest.mark.parametrize("bas,nw,seeds", [("STO-3G", 1, 24), ("STO-3G", 2, 12)])
+def test_shared_quartets_round_no_more_often(bas, nw, seeds):
+    """The accumulator's roundings (2^-44, uniform) of a build in which nothing is screened, against the oracle's 64-bit
+    sums: no larger than independent roundings of each quartet's distinct elements."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from quick_b200.get2e import Get2e
+    err2 = bound2 = 0.0
+    for seed in range(seeds):
+        b = build_basis(water_cluster(nw, 6.0, seed=50 + seed), bas)
+        rng = np.random.default_rng(seed)
+        X = rng.normal(size=(b.nbasis, b.nbasis)) * 0.3
+        D = X @ X.T
+        orc = O.Oracle(b)
+        Y, cp = orc.schwarz()
+        want, _ = orc.get2e(D, orc.density_cutoff(D), Y, cp, 1e-18, 1e-20)
+        eng = Get2e(b, integral_cutoff=1e-18, prim_limit=1e-20, schwarz=(Y, cp))
+        got = eng.fock2e(torch.tensor(D, device="cuda")).cpu().numpy()
+        eng.close()
+        N = _rounded_elements(b)
+        var = N + N.T + 2.0 * np.diag(np.diag(N))   # G = A + A^T: a diagonal element is doubled
+        err2 += np.sum((got - want) ** 2)
+        bound2 += var.sum() * 2.0 ** -88 / 12.0
+    assert err2 <= bound2, (err2 ** 0.5, bound2 ** 0.5)
