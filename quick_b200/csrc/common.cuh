@@ -367,5 +367,7 @@ inline std::vector<double> boys_table(const std::vector<long double>& grid) {
 
 // The tables above in a device's memory (get2e.cu).
 cudaError_t device_boys_tables(int device, cudaStream_t s, const double** tab, const double** rows);
+// Gives the device memory that the one-electron calls keep back to the driver (oei.cu).
+void oei_give_back(int device);
 
 }  // namespace qk

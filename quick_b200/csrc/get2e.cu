@@ -2458,6 +2458,7 @@ cudaError_t device_boys_tables(int device, cudaStream_t s, const double** tab, c
     *rows = tables[device] + rows_at;
     return cudaSuccess;
 }
+static std::atomic<int> g_contexts[64];   // live ones, per device
 }  // namespace qk
 
 extern "C" {
@@ -2496,6 +2497,7 @@ qk_ctx* qk_create(int device, int* status) {
         if (status) *status = fail(QK_ERR_CUDA, "Boys table upload failed");
         return nullptr;
     }
+    ++g_contexts[device];
     if (status) *status = QK_OK;
     return c;
 }
@@ -2512,7 +2514,9 @@ int qk_destroy(qk_ctx* c) {
         if (e) cudaEventDestroy(e);
     if (c->fork_ev) cudaEventDestroy(c->fork_ev);
     cudaStreamDestroy(c->stream);
+    const int device = c->device;
     delete c;
+    if (--g_contexts[device] == 0) oei_give_back(device);
     return QK_OK;
 }
 

@@ -452,13 +452,13 @@ static cudaStream_t oei_stream(int device) {
 
 // Per device, made at the first call and kept: a memory pool of its own for the calls'
 // work buffers, which keeps up to 256 MB between calls instead of giving the pages back
-// to the driver at every synchronisation.
+// to the driver at every synchronisation.  They go back with the device's last context.
+static std::mutex g_pool_mu;
+static cudaMemPool_t g_pools[64] = {};
 static cudaMemPool_t oei_pool(int device) {
-    static std::mutex mu;
-    static cudaMemPool_t pools[64] = {};
     if (device < 0 || device >= 64) return nullptr;
-    std::lock_guard<std::mutex> g(mu);
-    if (!pools[device]) {
+    std::lock_guard<std::mutex> g(g_pool_mu);
+    if (!g_pools[device]) {
         cudaMemPoolProps props{};
         props.allocType = cudaMemAllocationTypePinned;
         props.location.type = cudaMemLocationTypeDevice;
@@ -470,9 +470,13 @@ static cudaMemPool_t oei_pool(int device) {
             cudaMemPoolDestroy(p);
             return nullptr;
         }
-        pools[device] = p;
+        g_pools[device] = p;
     }
-    return pools[device];
+    return g_pools[device];
+}
+void oei_give_back(int device) {
+    std::lock_guard<std::mutex> g(g_pool_mu);
+    if (g_pools[device]) cudaMemPoolTrimTo(g_pools[device], 0);   // blocks in use stay
 }
 
 }  // namespace qk

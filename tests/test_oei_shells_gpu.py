@@ -2,6 +2,8 @@
 where its block size and chunks change, s to f shells, against the oracle; and bases
 whose components are not in QUICK's order (the function-pair kernel) against it."""
 import copy
+import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -58,3 +60,30 @@ def test_oei_charge_beyond_the_range_adds_nothing():
     far = (np.array([[1e155, 0.0, 0.0], [0.0, -3e160, 1e158]]), np.array([1.0, -2.0]))
     for got, want in zip(oei(b, far), oei(b, None)):
         assert np.array_equal(got, want)
+
+
+_GIVE_BACK = """
+import torch
+from quick_b200.basis import build_basis
+from quick_b200.get2e import Get2e
+from quick_b200.molecules import water_cluster
+from quick_b200.scf import oei
+small, large = (build_basis(water_cluster(n, 24.0, seed=1), "6-31G*") for n in (1, 80))
+free = lambda: torch.cuda.mem_get_info(0)[0]
+eng = Get2e(small)
+oei(small, None)
+before = free()
+oei(large, None)     # 3 n^2 doubles and more: 64 MB
+kept = before - free()
+eng.close()
+assert kept >= 20 << 20, kept
+assert free() >= before, (kept, before - free())
+"""
+
+
+def test_oei_memory_goes_back_with_the_last_context():
+    """In a process of its own: any context that lives keeps the memory."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    r = subprocess.run([sys.executable, "-c", _GIVE_BACK], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
