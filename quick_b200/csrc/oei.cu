@@ -489,8 +489,12 @@ extern "C" int qk_oei_host(int device, int natom, const double* xyz, const doubl
     if (natom <= 0 || nbasis <= 0 || maxcontract <= 0 || !xyz || !Z || !ncontract || !itype || !aexp ||
         !dcoeff || !ncenter || !S || !T || !V || next < 0 || (next > 0 && (!ext_xyz || !ext_q)))
         return QK_ERR_INVALID_ARG;
-    for (int i = 0; i < 3 * nbasis; ++i)
-        if (itype[i] < 0 || itype[i] > kOeiLmax) return QK_ERR_UNSUPPORTED;
+    for (int i = 0; i < nbasis; ++i) {   // the kernels' arrays hold a function of degree kOeiLmax
+        const int* t = itype + 3 * (size_t)i;
+        for (int x = 0; x < 3; ++x)
+            if (t[x] < 0 || t[x] > kOeiLmax) return QK_ERR_UNSUPPORTED;
+        if (t[0] + t[1] + t[2] > kOeiLmax) return QK_ERR_UNSUPPORTED;
+    }
     for (int i = 0; i < nbasis; ++i)
         if (ncenter[i] < 1 || ncenter[i] > natom || ncontract[i] < 1 || ncontract[i] > maxcontract)
             return QK_ERR_INVALID_ARG;
@@ -517,7 +521,6 @@ extern "C" int qk_oei_host(int device, int natom, const double* xyz, const doubl
         std::vector<int> f0, Ls;
         for (int f = 0; f < nbasis && shells;) {
             const int L = itype[3 * f] + itype[3 * f + 1] + itype[3 * f + 2];
-            if (L > kOeiLmax) { shells = false; break; }
             const int nc = (L + 1) * (L + 2) / 2;
             if (f + nc > nbasis) { shells = false; break; }
             for (int k = 0; k < nc && shells; ++k) {

@@ -39,6 +39,25 @@ def test_status_strings_without_gpu():
     assert L.qk_max_l() >= 2
 
 
+@pytest.mark.parametrize("power", [(2, 2, 0), (3, 3, 3), (0, 1, 3), (4, 0, 0), (-1, 0, 0)])
+def test_one_electron_call_refuses_functions_above_f(power):
+    """By their degree, before anything is sent to a device: the kernels hold no more."""
+    import copy
+    import numpy as np
+    from quick_b200 import _native
+    if not os.path.exists(_native.LIB_PATH):
+        pytest.skip("library not built")
+    from quick_b200.basis import build_basis
+    from quick_b200.molecules import water_cluster
+    from quick_b200.scf import oei
+    b = copy.copy(build_basis(water_cluster(1, 3.0), "CC-PVTZ"))
+    b.itype = np.array(b.itype)
+    b.itype[:, 5] = power
+    with pytest.raises(_native.QuickError) as e:
+        oei(b)
+    assert e.value.status == 105   # QK_ERR_UNSUPPORTED
+
+
 def test_basis_layout_matches_reference_convention():
     """The kernels assume QUICK's Cartesian order and cons factors; the host checks
     them on upload.  Verify the basis builder produces exactly that layout."""
