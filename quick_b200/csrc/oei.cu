@@ -25,8 +25,6 @@
 namespace qk {
 
 constexpr int kOeiLmax = 3;              // per function (f)
-constexpr int kEj = kOeiLmax + 3;        // j up to l + 2 (kinetic)
-constexpr int kEt = 2 * kOeiLmax + 3;    // t up to i + j
 
 struct OeiArgs {
     int nbasis, maxcontract, ncharge;
@@ -74,12 +72,9 @@ __device__ __forceinline__ void unroll_up(Fn&& f) {
     }
 }
 
-// 1-D Hermite coefficients E[i][j][t], i <= li, j <= lj, for one Cartesian axis.
+// 1-D Hermite coefficients E[i][j][t], i <= li, j <= lj, t <= i + j, for one Cartesian axis.
 __device__ __forceinline__ void hermite_E(int li, int lj, double XPA, double XPB, double oo2p, double E0,
-                                          double E[kOeiLmax + 1][kEj][kEt]) {
-    for (int i = 0; i <= li; ++i)
-        for (int j = 0; j <= lj; ++j)
-            for (int t = 0; t < kEt; ++t) E[i][j][t] = 0.0;
+                                          double E[kOeiLmax + 1][kOeiLmax + 1][2 * kOeiLmax + 1]) {
     E[0][0][0] = E0;
     for (int i = 0; i <= li; ++i) {
         for (int j = 0; j <= lj; ++j) {
@@ -134,11 +129,12 @@ __global__ void __launch_bounds__(128) oei_st_kernel(OeiArgs a) {
             for (int x = 0; x < 3; ++x) {
                 const int i0 = a.itype[3 * mu + x], j0 = a.itype[3 * nu + x];
                 const double PA = -be / pz * AB[x], PB = al / pz * AB[x];
-                double row[kEj], prev[kEj];   // s(i, .) and s(i-1, .)
+                constexpr int NJ = kOeiLmax + 3;   // j up to l + 2
+                double row[NJ], prev[NJ];   // s(i, .) and s(i-1, .)
                 row[0] = 1.0;
                 for (int j = 1; j <= j0 + 2; ++j) row[j] = PB * row[j - 1] + (j > 1 ? (j - 1) * oo2p * row[j - 2] : 0.0);
                 for (int i = 0; i < i0; ++i) {
-                    double next[kEj];
+                    double next[NJ];
                     for (int j = 0; j <= j0 + 2; ++j)
                         next[j] = PA * row[j] + oo2p * ((i ? i * prev[j] : 0.0) + (j ? j * row[j - 1] : 0.0));
                     for (int j = 0; j <= j0 + 2; ++j) { prev[j] = row[j]; row[j] = next[j]; }
@@ -177,7 +173,7 @@ __global__ void oei_kernel(OeiArgs a, int chunk, double* __restrict__ Vpart) {
     const double* B = a.xyz + 3 * (a.ncenter[nu] - 1);
     const int Lsum = la[0] + la[1] + la[2] + lb[0] + lb[1] + lb[2];
     double v = 0.0;
-    double E[3][kOeiLmax + 1][kEj][kEt];
+    double E[3][kOeiLmax + 1][kOeiLmax + 1][2 * kOeiLmax + 1];
     for (int p = 0; p < a.ncontract[mu]; ++p) {
         const double al = a.aexp[p + a.maxcontract * mu];
         const double ca = a.dcoeff[p + a.maxcontract * mu];
