@@ -85,6 +85,7 @@ struct DevData {
     double cut, primLimit;
     int boys_mode;                       // qk_set_boys: 0 accurate; 1 QUICK CPU order; 2 QUICK GPU order
     int exchange_only;                   // 1: the K part alone (the spin-density half of a UHF build)
+    int round_once;                      // 1: exchange blocks of a pair with itself are rounded together
 };
 
 __device__ __forceinline__ void atomic_fixed(unsigned long long* addr, double v) {
@@ -316,13 +317,10 @@ __device__ __forceinline__ void fock_quartet(const DevData& d, const double2* __
             for (int e = 0; e < ND; ++e) atomic_fixed(A + (size_t)(fc + c) * n + fd + e, wJ * jcd[c * ND + e]);
     }
     // Two exchange blocks of a quartet fall on the same elements where its pair is a shell
-    // with itself.  They are added before they are rounded: rounded one by one the two, which
-    // are often equal, would carry the same error twice.  That more than makes up for the bra's
-    // Coulomb block, rounded once per item, which has fewer kets where lanes share a quartet:
-    // error of G against 64 bits (2-norm) of one water in STO-3G 5.1e-14 with 32 kets an item
-    // and four blocks, 5.3e-14 with the shared lanes and four blocks, 3.8e-14 now; of two waters
-    // 8.5e-14, 9.0e-14, 7.0e-14.  Fewer atomics, too: 32 H2O / 6-31G* 10.87 -> 10.75 ms.
-    const bool ab1 = La == Lb && fa == fb, cd1 = Lc == Ld && fc == fd;
+    // with itself.  In the smallest molecules they are added before they are rounded:
+    // rounded one by one the two, which are often equal, carry the same error twice
+    // (lane_split).
+    const bool ab1 = La == Lb && fa == fb && d.round_once, cd1 = Lc == Ld && fc == fd && d.round_once;
     if constexpr (La == Lb)
         if (ab1) {
 #pragma unroll
@@ -1404,6 +1402,7 @@ static double cons_expected(const int c[3]) {
     return 1.0;
 }
 
+constexpr int kFewShells = 10;   // molecules of so few s, p, d and f shells: lane_split's first tier
 static DevData make_devdata(qk_ctx* c) {
     DevData d{};
     d.nbasis = c->nbasis;
@@ -1432,6 +1431,7 @@ static DevData make_devdata(qk_ctx* c) {
     d.cut = c->integralCutoff;
     d.primLimit = c->primLimit;
     d.boys_mode = c->boys_mode;
+    d.round_once = (int)c->qsh.size() <= kFewShells;
     return d;
 }
 
@@ -1641,8 +1641,15 @@ static int finish_work(qk_ctx* c);
 //   32 H2O / 6-31G* * 11.7 11.7 12.0 12.5 14.9 (pppp alone 0.164 0.113 0.113 0.105 0.134)
 // By the operations instead of the order, the long d classes alone are cut finer: dppp of
 // 10 H2O 0.105 -> 0.087, of the late cycle 0.201 -> 0.177.
+// An item has fewer kets where lanes share, and the bra's Coulomb block is rounded to the
+// accumulator once per item: for the smallest molecules (two kets an item) that raised the
+// error of G against 64 bits (2-norm) from 5.1e-14 to 5.3e-14 for one water in STO-3G and
+// from 8.5e-14 to 9.0e-14 for two.  There the exchange blocks of a pair with itself are
+// added before they are rounded (round_once): 3.8e-14 and 7.0e-14.  Done everywhere it would
+// lower the error everywhere (eight waters 2.2e-13 -> 2.0e-13), but move every G by its
+// roundings: 1.3e-8 of a late cycle's small G.  Larger molecules keep their bits.
 static int lane_split(int bnp, int knp, double prim_flops, int nq) {
-    const int chain = nq <= 10 ? 9 : nq <= 64 ? 40 : nq <= 256 ? 108 : 216;
+    const int chain = nq <= kFewShells ? 9 : nq <= 64 ? 40 : nq <= 256 ? 108 : 216;
     // a primitive quartet takes a lane about 0.35 us + 1.1 ns per operation
     const int limit = std::max((int)(chain * 0.41 / (0.35 + 1.1e-3 * prim_flops)), 1);
     int lb = 0, len = bnp;
