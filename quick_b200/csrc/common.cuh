@@ -87,7 +87,8 @@ __device__ __forceinline__ void boys_scaled(double T, double scale, const double
 // with the line at 36 for every M the second one needed an exponential and a division
 // and the evaluation was 47% of psss's instructions and 52% of its FP64 ones.
 //   M = 0: 48-byte rows, the six coefficients of F_0's Chebyshev interpolation on
-//          intervals of 1/32 (truncation 1.7e-16 relative); no exponential is needed.
+//          intervals of 1/32 (truncation 4.9e-17 relative, with all roundings at most
+//          2.8e-16); no exponential is needed.
 //   M > 0: 80-byte rows, F_{M+j}(T_k)/(j! (2M-1)!!) for j = 0..6 (Taylor, spacing 0.05) and
 //          exp(-T_k) for the downward recursion; the last two words are padding.
 // Both strides are odd multiples of 16 bytes: 32 lanes on random rows then spread over

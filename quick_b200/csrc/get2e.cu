@@ -9,8 +9,8 @@
 //    Schwarz test of a bra pair against a bucket is a prefix and every lane of a
 //    warp runs the same primitive loop;
 //  * one warp per work item = (bra pair, up to 32 consecutive ket pairs), one
-//    lane per shell quartet, straight-line HGP VRR/HRR generated per class
-//    (gen_eri.py), FP64 throughout;
+//    lane per shell quartet (in small molecules several, lane_split), straight-line
+//    HGP VRR/HRR generated per class (gen_eri.py), FP64 throughout;
 //  * J/K digestion into a full int64 fixed-point accumulator A (scale 2^44):
 //    J over the bra is warp-reduced before its atomics; G = A + A^T at the end.
 //    Integer addition is exact and order independent, so the Fock matrix is
@@ -1568,8 +1568,6 @@ static int upload_pairs(qk_ctx* c) {
     return QK_OK;
 }
 
-// Work items of every class: (bra pair, first ket, count) chunks of <= 32
-// kets that pass the Schwarz test, unique quartets only.
 // Launch shape of class ci for the context's current work list: warps per block
 // (tuned or default), the matching dynamic shared memory (cooperative classes:
 // one work area per warp), and a persistent grid of as many blocks as can be
@@ -1589,7 +1587,8 @@ static cudaError_t occupancy(int device, int ci, int part, int wpb, size_t smem,
     // The per-lane kernels use no shared memory and live on L1 (psss is 17% slower at the
     // largest shared carveout), but beside the cooperative classes an SM keeps their
     // carveout unless a kernel asks for its own: 32 H2O / 6-31G* over four streams
-    // 12.71 ms without the request, 11.23 with it.
+    // 12.71 ms without the request, 11.23 with it.  Only these kernels ask: the batched
+    // ones and the merged s/p one do not, and it was not measured for them.
     if (e == cudaSuccess && !g_classes[ci].coop)
         e = cudaFuncSetAttribute(g_classes[ci].kernel(part == 1), cudaFuncAttributePreferredSharedMemoryCarveout,
                                  cudaSharedmemCarveoutMaxL1);
@@ -1633,14 +1632,15 @@ static int finish_work(qk_ctx* c);
 // class's time and lanes share it; the price is a digestion by one lane of each group.
 // The limit on the chain falls with the class's cost per primitive quartet and follows
 // the number of shells, not the screened lists: lists built at different cutoffs are
-// cut alike.  Whole builds (ms, * one after another) without a limit, with this rule by
-// the class's order, and with limits of 54, 27 and 9 for every class:
-//   H2O / STO-3G 0.158 0.069 0.106 0.080 0.063    4 H2O / STO-3G 0.136 0.064 0.097 0.081 0.075
-//   10 H2O / 6-31G* 1.19 0.95 0.93 0.99 1.06
-//   20 H2O / 6-31G*, density of a late cycle * 3.36 2.29 2.35 2.38 2.77
-//   32 H2O / 6-31G* * 11.7 11.7 12.0 12.5 14.9 (pppp alone 0.164 0.113 0.113 0.105 0.134)
-// By the operations instead of the order, the long d classes alone are cut finer: dppp of
-// 10 H2O 0.105 -> 0.087, of the late cycle 0.201 -> 0.177.
+// cut alike.  Whole builds (ms over four streams, * one after another) without a limit, with
+// this rule and with limits of 54, 27 and 9 for every class:
+//   H2O / STO-3G 0.129 0.055 0.086 0.066 0.055    4 H2O / STO-3G 0.148 0.056 0.103 0.078 0.070
+//   10 H2O / 6-31G* 1.21 0.864 0.862 0.889 0.985
+//   20 H2O / 6-31G*, density of a late cycle * 2.22 1.86 1.90 1.99 2.43
+//   32 H2O / 6-31G* * 10.95 10.87 11.13 11.65 13.87 (pppp alone 0.152 0.101 0.103 0.099 0.125)
+//   16 H2O / 6-31G**, mixed form * 4.15 3.77 3.83 3.92 4.38    3 H2O / cc-pVTZ 3.08 2.01 2.09 2.07 2.02
+// A class with few quartets in a large molecule is treated as the rest: dppp of 10 H2O takes
+// 0.084 and 0.068 with a limit of 9, of the late cycle 0.164 and 0.121.
 // An item has fewer kets where lanes share, and the bra's Coulomb block is rounded to the
 // accumulator once per item: for the smallest molecules (two kets an item) that raised the
 // error of G against 64 bits (2-norm) from 5.1e-14 to 5.3e-14 for one water in STO-3G and

@@ -100,7 +100,7 @@ __device__ __forceinline__ void hermite_E(int li, int lj, double XPA, double XPB
 }
 
 // Gaussian products beyond this exponent (exp(-75) = 2.7e-33) contribute nothing that
-// a 64-bit sum could show.
+// a 64-bit sum could show; an element that has no others is 0.
 constexpr double kOeiExpMax = 75.0;
 
 // Overlap and kinetic energy of one function pair per thread, from the 1-d overlaps
@@ -297,8 +297,8 @@ __device__ __forceinline__ void hermite_E_fixed(double XPA, double XPB, double o
 // sums in a fixed order.  A charge costs its Boys function and the R recursion (about
 // 60 + 3 NT operations); the reduction, 10 NT shuffles a warp, is small beside the
 // 32 charges a thread has of 4000.  All threads work on one primitive pair, so a pair
-// whose Gaussian product vanishes is left out by the whole block (70% of them for
-// twenty waters).  20 H2O / 6-31G* with 4000 charges, whole call: 2.2 ms, against 12.2
+// whose Gaussian product vanishes is left out by the whole block (52 to 55% of them for
+// twenty waters).  20 H2O / 6-31G* with 4000 charges, whole call: 2.0 ms, against 12.2
 // with a thread per shell pair that contracted charge by charge and a thread per
 // function pair for the nuclei.
 template <int LA, int LB>

@@ -1,9 +1,10 @@
 """GPU test of the device Boys function F_m(T) against high-precision values.
 
-The Fock kernels evaluate F_0..F_M in two forms: the per-lane kernels by a 7-term
-Taylor step from a 0.05-spaced table below T = 36 then downward recursion, the
-asymptotic form with upward recursion above it (boys_scaled_rows); the
-cooperative kernels one m at a time (boys_one).  The oracle uses the same
+The Fock kernels evaluate F_0..F_M in two forms: the per-lane kernels from tables
+that reach to T = 36 (M = 0) .. 71 (M = 12), a Chebyshev fit of F_0 or a 7-term
+Taylor step (0.05-spaced) and downward recursion, and the asymptotic form alone
+above them (boys_scaled_rows); the cooperative kernels one m at a time by a Taylor
+step below T = 36 and upward recursion above it (boys_one).  The oracle uses a
 tabulated method, so a table error common to both would pass the Fock parity
 tests; this test pins the device values to mpmath directly (1F1 at 40 digits),
 1e-13 relative, for m = 0..12 (ffff quartets need M = 12) and T in [0, 36) and
