@@ -339,8 +339,8 @@ int qk_sp2_run(double *Ya_dev, double *Yb_dev, double *Y2_dev, int n, double noc
  * ncenter(nbasis) 1-based.  Charges: nuclei Z(natom) at xyz(3,natom) plus `next`
  * external point charges ext_q at ext_xyz(3,next) (QM/MM).  Writes S, T, V
  * (nbasis^2, symmetric) to host arrays; functions up to f.  The calls keep up to 256 MB
- * of device memory per device for the next one, outside any context's figures; it goes
- * back when the last context on the device is destroyed. */
+ * of device memory per device for the next one, outside any context's figures; all but
+ * 32 MB of it goes back when the last context on the device is destroyed. */
 int qk_oei_host(int device, int natom, const double *xyz, const double *Z, int nbasis,
                 int maxcontract, const int *ncontract, const int *itype, const double *aexp,
                 const double *dcoeff, const int *ncenter, int next, const double *ext_xyz,
